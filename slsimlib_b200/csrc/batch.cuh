@@ -52,7 +52,24 @@ struct Chunk {
 // distinct banks).  Keeping them out of registers leaves the tree walk the
 // registers it needs.
 constexpr int kBatchSmemDoubles = 22;
-inline size_t batch_smem_bytes(int block) { return (size_t)kBatchSmemDoubles * block * sizeof(double); }
+// The kernel's form: GLB_PREC_SPLIT, GLB_PREC_FP64 (the node-at-a-time walk:
+// batches with NFW haloes, see launch_plane_steps) or kStripForm (the strip
+// walk: every other FP64 batch).
+constexpr int kStripForm = 3;
+int batch_form(const std::vector<glb_lens *> &lenses, int precision) {
+  if (precision == GLB_PREC_SPLIT) return precision;
+  for (const glb_lens *l : lenses)
+    if (l->has_nfw) return GLB_PREC_FP64;
+  return kStripForm;
+}
+// The strip form adds the strip walk's: a StripWarp per warp and the
+// exponential's table.
+inline size_t batch_smem_bytes(int block, int form) {
+  size_t b = (size_t)kBatchSmemDoubles * block * sizeof(double);
+  if (form == kStripForm)
+    b += (size_t)(block / 32) * sizeof(StripWarp) + sizeof(ExpTab);
+  return b;
+}
 
 // LensPlaneSingular::force for one plane (planes.cpp:114-161): the plane's
 // halos summed into f[c * stride] = {alpha0, alpha1, kappa, gamma0, gamma1};
@@ -60,7 +77,7 @@ inline size_t batch_smem_bytes(int block) { return (size_t)kBatchSmemDoubles * b
 template <int PREC>
 __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *halos, const NFWTables *tab,
                                             double xx0, double xx1, bool valid, double *f, double *h,
-                                            int stride) {
+                                            int stride, StripWarp *W, const ExpTab *etab) {
   for (int c = 0; c < 5; ++c) f[c * stride] = 0.0;
   for (int k = 0; k < P.nhalo; ++k) {
     const HaloDev *H = halos + P.halo0 + k;
@@ -68,7 +85,10 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
     double a[5];
     if (H->kind == HALO_PARTICLES) {
       for (int c = 0; c < 5; ++c) h[c] = 0.0;
-      particle_halo_acc<PREC, false, false, true>(H->tree, xc0, xc1, valid, h);
+      if constexpr (PREC == kStripForm)
+        particle_halo_f64<false>(H->tree, xc0, xc1, valid, *W, *etab, h, 1);
+      else
+        particle_halo_acc<PREC, false, true>(H->tree, xc0, xc1, valid, h);
       // force_halo negates the walk's alpha (particle_halo.h:432-433)
       a[0] = -h[0];
       a[1] = -h[1];
@@ -105,12 +125,20 @@ template <int PREC>
 __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
                                                NFWTables tab, const double *xs, const unsigned *outidx,
                                                double *y, double *A, int *counter) {
-  extern __shared__ double bsm[];
+  extern __shared__ __align__(16) double bsm[];
   const int lane = threadIdx.x & 31;
   const int B = blockDim.x;
   double *st = bsm + threadIdx.x;          // st[c * B], c = 0..11
   double *f = bsm + 12 * B + threadIdx.x;  // f[c * B], c = 0..4
   double *h = bsm + 17 * B + 5 * threadIdx.x;  // h[0..4]
+  StripWarp *W = nullptr;
+  ExpTab *etab = nullptr;
+  if constexpr (PREC == kStripForm) {
+    W = reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
+    etab = reinterpret_cast<ExpTab *>(reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + B / 32);
+    strip_exp_table(*etab);
+    __syncthreads();
+  }
   for (;;) {
     int c = 0;
     if (lane == 0) c = atomicAdd(counter, 1);
@@ -168,7 +196,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchun
       const bool v = valid && j < jmax;
       {
         const PlaneDev &P = L.planes[j];
-        plane_force<PREC>(P, L.halos, &tab, st[0] * P.Dphys, st[B] * P.Dphys, v, f, h, B);
+        plane_force<PREC>(P, L.halos, &tab, st[0] * P.Dphys, st[B] * P.Dphys, v, f, h, B, W, etab);
       }
       if (v) {
         // include/lens.h:1027-1066, the state reloaded from shared memory
@@ -247,17 +275,34 @@ int make_lens_dev(glb_lens *l, LensDev &d) {
   return 0;
 }
 
-int persistent_grid(int block, int precision, int *grid) {
+int persistent_grid(int block, int form, int *grid) {
   int dev = 0, sms = 0, per_sm = 0;
   CKR(cudaGetDevice(&dev));
   CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (precision == GLB_PREC_SPLIT)
-    CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<GLB_PREC_SPLIT>, block,
-                                                      batch_smem_bytes(block)));
-  else
-    CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<GLB_PREC_FP64>, block,
-                                                      batch_smem_bytes(block)));
+  const void *k = form == GLB_PREC_SPLIT ? (const void *)k_batch<GLB_PREC_SPLIT>
+                  : form == kStripForm   ? (const void *)k_batch<kStripForm>
+                                         : (const void *)k_batch<GLB_PREC_FP64>;
+  if (form == kStripForm)  // more than the default 48 KB
+    CKR(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes(256, form)));
+  CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, batch_smem_bytes(block, form)));
   *grid = sms * std::max(per_sm, 1);
+  return 0;
+}
+
+int launch_batch(int form, int grid, int block, cudaStream_t s, const Chunk *chunks, int nchunks,
+                 const LensDev *lenses, const NFWTables &tab, const double *xs, const unsigned *outidx, double *y,
+                 double *A, int *counter) {
+  const size_t smem = batch_smem_bytes(block, form);
+  if (form == GLB_PREC_SPLIT)
+    k_batch<GLB_PREC_SPLIT><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+  else if (form == kStripForm)
+    k_batch<kStripForm><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+  else
+    k_batch<GLB_PREC_FP64><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess)
+    return fail(GLB_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e) + " launching k_batch with block " +
+                                  std::to_string(block) + " grid " + std::to_string(grid));
   return 0;
 }
 
@@ -267,7 +312,7 @@ int persistent_grid(int block, int precision, int *grid) {
 struct glb_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
-  int precision = GLB_PREC_FP64;
+  int form = GLB_PREC_FP64;  // k_batch's
   int block = 128, grid = 0;
   std::vector<glb_lens *> lenses;
   std::vector<size_t> n1d, offset;
@@ -333,17 +378,8 @@ void drop_graph(glb_batch *b) {
 int batch_enqueue(glb_batch *b) {
   (void)cudaGetLastError();  // launch errors below are this launch's own
   CKR(cudaMemsetAsync(b->counter.p, 0, sizeof(int), b->stream));
-  if (b->precision == GLB_PREC_SPLIT)
-    k_batch<GLB_PREC_SPLIT><<<b->grid, b->block, batch_smem_bytes(b->block), b->stream>>>(b->d_chunks.p, b->nchunks, b->d_lenses.p, b->tab,
-                                                                 nullptr, nullptr, b->y.p, b->A.p, b->counter.p);
-  else
-    k_batch<GLB_PREC_FP64><<<b->grid, b->block, batch_smem_bytes(b->block), b->stream>>>(b->d_chunks.p, b->nchunks, b->d_lenses.p, b->tab,
-                                                                nullptr, nullptr, b->y.p, b->A.p, b->counter.p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return fail(GLB_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e) + " launching k_batch with block " +
-                                  std::to_string(b->block) + " grid " + std::to_string(b->grid));
-  return 0;
+  return launch_batch(b->form, b->grid, b->block, b->stream, b->d_chunks.p, b->nchunks, b->d_lenses.p, b->tab, nullptr,
+                      nullptr, b->y.p, b->A.p, b->counter.p);
 }
 }  // namespace
 
@@ -359,7 +395,6 @@ int glb_batch_create_grids(glb_lens *const *lenses, int nlens, const size_t *n1d
   CKR(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   CKR(cudaEventCreate(&b->e0));
   CKR(cudaEventCreate(&b->e1));
-  b->precision = precision;
   std::vector<LensDev> L(nlens);
   for (int i = 0; i < nlens; ++i) {
     if (!lenses[i]) return fail(GLB_ERR_ARG, "null lens");
@@ -382,7 +417,8 @@ int glb_batch_create_grids(glb_lens *const *lenses, int nlens, const size_t *n1d
   CKR(cudaMemcpy(b->d_lenses.p, L.data(), nlens * sizeof(LensDev), cudaMemcpyHostToDevice));
   if (int rc = batch_chunks(b.get(), 3)) return rc;
   if (int rc = device_nfw_tables(b->tab)) return rc;
-  if (int rc = persistent_grid(b->block, precision, &b->grid)) return rc;
+  b->form = batch_form(b->lenses, precision);
+  if (int rc = persistent_grid(b->block, b->form, &b->grid)) return rc;
   *out = b.release();
   return 0;
 }
@@ -435,7 +471,7 @@ int glb_batch_autotune(glb_batch *b, int *best_block, double *best_ms) {
   int bb = b->block, bg = b->grid;
   for (int c : {64, 128, 256}) {
     b->block = c;
-    if (int rc = persistent_grid(c, b->precision, &b->grid)) return rc;
+    if (int rc = persistent_grid(c, b->form, &b->grid)) return rc;
     double t;
     if (int rc = time_it(&t)) return rc;
     if (t < best) {
@@ -481,7 +517,7 @@ int glb_batch_set_block(glb_batch *b, int block) {
   if (!b || (block != 64 && block != 128 && block != 256)) return fail(GLB_ERR_ARG, "block must be 64, 128 or 256");
   if (int rc = set_dev(b->device)) return rc;
   b->block = block;
-  if (int rc = persistent_grid(block, b->precision, &b->grid)) return rc;
+  if (int rc = persistent_grid(block, b->form, &b->grid)) return rc;
   drop_graph(b);
   return 0;
 }
@@ -600,6 +636,7 @@ struct Slot {
 struct glb_server {
   int device = 0;
   int precision = GLB_PREC_FP64;
+  int form = GLB_PREC_FP64;  // k_batch's
   size_t cap = 0;  // rays per batch at most (max_rays_per_batch; the pinned staging of a slot)
   size_t reserve = 0;  // device bytes admission leaves free for everything else
   size_t total_bytes = 0;
@@ -758,13 +795,9 @@ int launch_slot(glb_server *S, Slot &sl) {
   CKR(cudaMemcpyAsync(dch, C.data(), C.size() * sizeof(Chunk), cudaMemcpyHostToDevice, s));
   CKR(cudaMemsetAsync(counter, 0, sizeof(int), s));
   if (!C.empty()) {
-    if (S->precision == GLB_PREC_SPLIT)
-      k_batch<GLB_PREC_SPLIT><<<S->grid, 128, batch_smem_bytes(128), s>>>(dch, (int)C.size(), S->d_lenses.p, S->tab,
-                                                                         dxs, perm, dy, dA, counter);
-    else
-      k_batch<GLB_PREC_FP64><<<S->grid, 128, batch_smem_bytes(128), s>>>(dch, (int)C.size(), S->d_lenses.p, S->tab,
-                                                                        dxs, perm, dy, dA, counter);
-    CKR(cudaGetLastError());
+    if (int rc = launch_batch(S->form, S->grid, 128, s, dch, (int)C.size(), S->d_lenses.p, S->tab, dxs, perm, dy, dA,
+                              counter))
+      return rc;
   }
   // large requests: the lens path's per-plane kernels over the request's rays
   // (contiguous in sorted order), results scattered to their batch slots
@@ -942,7 +975,8 @@ int glb_server_create(glb_lens *const *models, int nmodels, size_t max_rays_per_
   CKR(S->d_lenses.alloc(nmodels));
   CKR(cudaMemcpy(S->d_lenses.p, L.data(), nmodels * sizeof(LensDev), cudaMemcpyHostToDevice));
   if (int rc = device_nfw_tables(S->tab)) return rc;
-  if (int rc = persistent_grid(128, precision, &S->grid)) return rc;
+  S->form = batch_form(S->models, precision);
+  if (int rc = persistent_grid(128, S->form, &S->grid)) return rc;
   size_t cap = S->cap;
   for (int i = 0; i < nslots; ++i) {
     auto sl = std::make_unique<Slot>();

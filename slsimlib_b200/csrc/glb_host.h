@@ -59,6 +59,8 @@ struct Tree {
   TreeDev dev{};
   DBuf<GNode> nodes;
   DBuf<GNodeS> snodes;
+  DBuf<TNode> tnodes;
+  DBuf<FNode> fnodes;
   DBuf<float4> parts;
   DBuf<float4> prel;
   DBuf<float4> bigs;

@@ -53,7 +53,23 @@ struct __align__(16) GNodeS {
   int skip, leaf, start, count;  // leaf: particle range; internal: big-particle range
 };
 
+// The node rows of the FP64 strip walk (walk_strip.cuh), split by use: what a
+// lane reads to classify its node (32 bytes, consecutive over a warp) and the
+// rest of the far-field term (32 bytes; mass and quadrupole divided by pi,
+// q1 = -q0).
+struct __align__(16) TNode {
+  double cx, cy;   // centre
+  float olo, ohi;  // open2 less and plus the classification's margin
+  int skip;
+  int info;        // 1: leaf, 2: internal with softened particles, 0: neither
+};
+struct __align__(16) FNode {
+  double mpi, q0pi, q2pi, pad;
+};
+
 struct TreeDev {
+  const TNode *tnodes;
+  const FNode *fnodes;
   const GNode *nodes;
   const GNodeS *snodes;
   const float4 *parts;  // sorted particles {x, y, mass, size}

@@ -27,6 +27,7 @@
 #include "walk_split.cuh"
 #include "walk_group.cuh"
 #include "walk_halos.cuh"
+#include "walk_strip.cuh"
 
 using namespace glb;
 
@@ -210,6 +211,7 @@ struct glb_lens {
   std::vector<PlaneHost> field;  // LensPlaneTree planes, in insertion order
   std::vector<PlaneHost *> planes;  // main and field planes in order of distance (combinePlanes)
   std::vector<char> plane_field;    // per plane: holds a field plane (HALO_FIELD)
+  bool has_nfw = false;             // any plane holds NFW haloes (or a field plane)
   std::vector<double> plane_z, Dl, dDl;  // combined, source pseudo-plane last
   bool toggle_source_plane = false;
   double zs_implant = 0;
@@ -408,28 +410,41 @@ __global__ void k_grid(size_t N1d, double c0, double c1, double range, double *x
   x[2 * i + 1] = c1 + range * (1.0 * (double)(i / N1d) / (double)(N1d - 1) - 0.5);
 }
 
-template <int PREC, bool PHI, bool COUNT = false, bool SKIPNEAR = false, bool MERGE = true>
+// A particle halo's tree force at (rx, ry), periodic images included; FP64 here
+// is the node-at-a-time walk (particle_halo_f64 is the strip walk).
+template <int PREC, bool COUNT = false, bool SKIPNEAR = false, bool MERGE = true>
 __device__ __forceinline__ void particle_halo_acc(const TreeDev &T, double rx, double ry, bool valid, double *acc,
                                                   WalkCount *wc = nullptr) {
-  if (T.periodic) {
-    // force2D_recur with a periodic buffer: nine shifted copies (quadTree.h:944-974)
-    for (int i = -1; i < 2; ++i)
-      for (int j = -1; j < 2; ++j) {
-        if (PREC == GLB_PREC_FP64)
-          walk_f64<PHI, COUNT>(T, rx + i * T.period_x, ry + j * T.period_y, valid, acc, wc);
-        else if (PREC == GLB_PREC_FP32)
-          walk_split<true>(T, rx + i * T.period_x, ry + j * T.period_y, valid, acc);
-        else
-          walk_split<false, SKIPNEAR, MERGE>(T, rx + i * T.period_x, ry + j * T.period_y, valid, acc);
-      }
-  } else {
-    if (PREC == GLB_PREC_FP64)
-      walk_f64<PHI, COUNT>(T, rx, ry, valid, acc, wc);
-    else if (PREC == GLB_PREC_FP32)
-      walk_split<true>(T, rx, ry, valid, acc);
-    else
-      walk_split<false, SKIPNEAR, MERGE>(T, rx, ry, valid, acc);
-  }
+  const int im = T.periodic ? 1 : 0;
+  // force2D_recur with a periodic buffer: nine shifted copies (quadTree.h:944-974)
+  for (int i = -im; i <= im; ++i)
+    for (int j = -im; j <= im; ++j) {
+      const double x = im ? rx + i * T.period_x : rx, y = im ? ry + j * T.period_y : ry;
+      if (PREC == GLB_PREC_FP64)
+        walk_f64<COUNT>(T, x, y, valid, acc, wc);
+      else if (PREC == GLB_PREC_FP32)
+        walk_split<true>(T, x, y, valid, acc);
+      else
+        walk_split<false, SKIPNEAR, MERGE>(T, x, y, valid, acc);
+    }
+}
+
+// The shared memory of a block's strip walks (walk_strip.cuh).
+template <int B>
+struct StripBlock {
+  ExpTab tab;
+  StripWarp warp[B / 32];
+};
+
+// The same in the plain FP64 form: the strip walk, per periodic image.
+// acc[c * A], c = 0..4 (5 with PHI).
+template <bool PHI>
+__device__ __forceinline__ void particle_halo_f64(const TreeDev &T, double rx, double ry, bool valid, StripWarp &W,
+                                                  const ExpTab &tab, double *acc, int A) {
+  const int im = T.periodic ? 1 : 0;
+  for (int i = -im; i <= im; ++i)
+    for (int j = -im; j <= im; ++j)
+      walk_strip<PHI>(T, im ? rx + i * T.period_x : rx, im ? ry + j * T.period_y : ry, valid, W, tab, acc, A);
 }
 
 // Analytic halo of a plane at one position; kept out of line so that the rare
@@ -526,6 +541,7 @@ __device__ __forceinline__ void recursion_step(const StepArgs &a, size_t k, doub
 
 // One lens plane for every ray: LensPlaneSingular::force + the recursion of
 // include/lens.h:1003-1066.
+// (split form, and the node-at-a-time FP64 walk)
 template <int PREC, bool COUNT = false, bool FIELD = false>
 __device__ __forceinline__ void plane_step(const StepArgs &a) {
   const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -557,14 +573,14 @@ __device__ __forceinline__ void plane_step(const StepArgs &a) {
     if (kind == HALO_PARTICLES) {
       if (COUNT) {
         WalkCount wc;
-        particle_halo_acc<PREC, false, true>(H->tree, xc0, xc1, valid, acc, &wc);
+        particle_halo_acc<PREC, true>(H->tree, xc0, xc1, valid, acc, &wc);
         unsigned long long v[7] = {wc.V, wc.F, wc.P, wc.B, wc.S, wc.Wn, wc.Wp};
         for (int c = 0; c < 7; ++c) {
           for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(kFull, v[c], o);
           if ((threadIdx.x & 31) == 0) atomicAdd(a.counts + c, v[c]);
         }
       } else {
-        particle_halo_acc<PREC, false>(H->tree, xc0, xc1, valid, acc);
+        particle_halo_acc<PREC>(H->tree, xc0, xc1, valid, acc);
       }
       // LensHaloParticles::force_halo negates alpha (particle_halo.h:432-433)
       acc[0] = -acc[0];
@@ -630,15 +646,71 @@ __device__ __forceinline__ void plane_step(const StepArgs &a) {
   st[11 * n + k] = s3;
 }
 
-// The FP64 form keeps the compiler's own register choice; the split form is
-// latency-bound (dependent node loads and short arithmetic chains), and
-// capping it at 64 registers (8 blocks of 128 per SM, half the warp slots)
-// buys the occupancy that hides them, spills included.
-// Planes holding a field plane (HALO_FIELD) use the FIELD instances, so that
-// the halo-tree walk adds no code to the kernels of particle planes.
-template <int PREC, bool COUNT = false, bool FIELD = false>
+// The split form is latency-bound (dependent node loads and short arithmetic
+// chains), and capping it at 64 registers (8 blocks of 128 per SM, half the
+// warp slots) buys the occupancy that hides them, spills included.  Planes
+// holding a field plane (HALO_FIELD) use the FIELD instances, so that the
+// halo-tree walk adds no code to the kernels of particle planes.
+template <bool COUNT, bool FIELD>
 __global__ void __launch_bounds__(128) k_plane_step(StepArgs a) {
-  plane_step<PREC, COUNT, FIELD>(a);
+  plane_step<GLB_PREC_FP64, COUNT, FIELD>(a);
+}
+
+// FP64 plane step: the plane's halos in insertion order, particle halos by the
+// strip walk, then the recursion.  ONE: the plane holds one particle halo, its
+// tree in the kernel parameters (a.tree), so that the walk's pointers and
+// scalars are constant operands.
+template <bool ONE>
+__global__ void __launch_bounds__(128, 5) k_plane_step_f64(const __grid_constant__ StepArgs a) {
+  __shared__ StripBlock<128> S;
+  __shared__ double sacc[5 * 128];
+  const int t = threadIdx.x;
+  strip_exp_table(S.tab);
+  __syncthreads();
+  const size_t k = blockIdx.x * (size_t)blockDim.x + t;
+  const bool inrange = k < a.n;
+  const int jmax = (a.jmax_ray && inrange) ? a.jmax_ray[k] : a.jmax;
+  const bool valid = inrange && a.j < jmax;
+  if (!__any_sync(kFull, valid)) return;
+  double *acc = sacc + t;
+  if (ONE) {
+    const double D = a.planes[a.j].Dphys;
+    for (int c = 0; c < 5; ++c) acc[c * 128] = 0.0;
+    particle_halo_f64<false>(a.tree, valid ? __dmul_rn(a.st[k], D) - a.tree_px : 0.0,
+                             valid ? __dmul_rn(a.st[a.n + k], D) - a.tree_py : 0.0, valid, S.warp[t >> 5], S.tab, acc,
+                             128);
+  }
+  const PlaneDev P = a.planes[a.j];
+  double xx0 = 0, xx1 = 0;
+  if (valid) {
+    xx0 = __dmul_rn(a.st[k], P.Dphys);
+    xx1 = __dmul_rn(a.st[a.n + k], P.Dphys);
+  }
+  double al0 = 0, al1 = 0, kap = 0, g0 = 0, g1 = 0;
+  for (int h = 0; h < P.nhalo; ++h) {
+    const HaloDev *H = a.halos + P.halo0 + h;
+    const double xc0 = xx0 - H->px, xc1 = xx1 - H->py;
+    if (H->kind == HALO_PARTICLES) {
+      if (!ONE) {
+        for (int c = 0; c < 5; ++c) acc[c * 128] = 0.0;
+        particle_halo_f64<false>(H->tree, xc0, xc1, valid, S.warp[t >> 5], S.tab, acc, 128);
+      }
+      // LensHaloParticles::force_halo negates alpha (particle_halo.h:432-433)
+      al0 += acc[0];
+      al1 += acc[128];
+      kap += acc[256];
+      g0 += acc[384];
+      g1 += acc[512];
+    } else if (valid) {
+      const Force5 f = analytic_halo(H, &a.tab, xc0, xc1);
+      al0 -= f.a0;
+      al1 -= f.a1;
+      kap += f.k;
+      g0 += f.g0;
+      g1 += f.g1;
+    }
+  }
+  if (valid) recursion_step(a, k, al0, al1, kap, g0, g1);
 }
 // Split-form plane step with the block-level group walk (walk_group.cuh) for
 // a plane holding exactly one particle halo (its tree in a.tree, a kernel
@@ -736,7 +808,11 @@ __global__ void __launch_bounds__(128, 8) k_plane_step_split(const __grid_consta
 // (analytic haloes; particle trees and field planes take no such argument).
 __global__ void __launch_bounds__(128) k_halo_force(HaloDev H, NFWTables tab, size_t n, const double *x,
                                                     double *out, int subtract = 0, double screening = 1.0) {
-  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  __shared__ StripBlock<128> S;
+  const int t = threadIdx.x;
+  strip_exp_table(S.tab);
+  __syncthreads();
+  const size_t k = blockIdx.x * (size_t)blockDim.x + t;
   const bool valid = k < n;
   if (!__any_sync(kFull, valid)) return;
   double x0 = 0, x1 = 0;
@@ -746,7 +822,7 @@ __global__ void __launch_bounds__(128) k_halo_force(HaloDev H, NFWTables tab, si
   }
   double acc[6] = {0, 0, 0, 0, 0, 0};
   if (H.kind == HALO_PARTICLES) {
-    particle_halo_acc<GLB_PREC_FP64, true>(H.tree, x0, x1, valid, acc);
+    particle_halo_f64<true>(H.tree, x0, x1, valid, S.warp[t >> 5], S.tab, acc, 1);
   } else if (H.kind == HALO_FIELD) {
     field_plane_acc<true>(H.htree, tab, x0, x1, valid, acc);
   } else if (valid && subtract) {
@@ -779,14 +855,29 @@ __device__ __forceinline__ void tree_force(const TreeDev &T, size_t n, const dou
     x1 = x[2 * k + 1];
   }
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  particle_halo_acc<PREC, false, false, false, false>(T, x0, x1, valid, acc);  // a flush per opened leaf
+  particle_halo_acc<PREC, false, false, false>(T, x0, x1, valid, acc);  // a flush per opened leaf
   if (!valid) return;
   for (int c = 0; c < 5; ++c) out[5 * k + c] = acc[c];
 }
 
-__global__ void __launch_bounds__(128) k_tree_force(const __grid_constant__ TreeDev T, size_t n, const double *x,
-                                                    double *out) {
-  tree_force<GLB_PREC_FP64>(T, n, x, out);
+__global__ void __launch_bounds__(128, 5) k_tree_force_f64(const __grid_constant__ TreeDev T, size_t n,
+                                                          const double *x, double *out) {
+  __shared__ StripBlock<128> S;
+  const int t = threadIdx.x;
+  strip_exp_table(S.tab);
+  __syncthreads();
+  const size_t k = blockIdx.x * (size_t)blockDim.x + t;
+  const bool valid = k < n;
+  if (!__any_sync(kFull, valid)) return;
+  double x0 = 0, x1 = 0;
+  if (valid) {
+    x0 = x[2 * k];
+    x1 = x[2 * k + 1];
+  }
+  double acc[5] = {0, 0, 0, 0, 0};
+  particle_halo_f64<false>(T, x0, x1, valid, S.warp[t >> 5], S.tab, acc, 1);
+  if (!valid) return;
+  for (int c = 0; c < 5; ++c) out[5 * k + c] = acc[c];
 }
 // the FP32-arithmetic forms, capped at 80 registers (6 blocks of 128 per SM) for occupancy
 template <int PREC>
@@ -1008,7 +1099,10 @@ void combine_planes(glb_lens *l) {
   for (size_t i = 0; i < n; ++i) l->plane_z[i] = l->planes[i]->z;
   l->plane_field.assign(n, 0);
   for (size_t i = 0; i < n; ++i)
-    for (const glb_halo *h : l->planes[i]->halos) l->plane_field[i] |= h->kind == HALO_FIELD;
+    for (const glb_halo *h : l->planes[i]->halos) {
+      l->plane_field[i] |= h->kind == HALO_FIELD;
+      l->has_nfw = l->has_nfw || h->kind == HALO_FIELD || h->kind == HALO_NFW;
+    }
   if (n > 0 && l->zsource <= l->plane_z[n - 1]) l->zsource = l->plane_z[n - 1] + 0.1;
   l->plane_z[n] = l->zsource;
   l->Dl[n] = coordist2(l->cosmo, 0, l->zsource);
@@ -1088,7 +1182,11 @@ int ensure_ws(LensWS *w, size_t n, bool per_ray) {
 // One launch per plane, in order.  Split-form planes that hold exactly one
 // particle halo and no field plane run the group walk (k_plane_step_split_g,
 // the tree in the kernel parameters); planes with a field plane use the FIELD
-// instances.
+// instances.  FP64 planes run the strip walk, except in lenses with NFW haloes
+// (field planes hold them): the NFW shear and deflection of the table's first
+// bin cancel up to 1e9-fold (nfw_g, nfw_g2), so a ray that meets a halo's
+// centre carries the last bit of its position into the ninth digit of A, and
+// those lenses keep the walk whose last bits are the reference's operations.
 constexpr size_t kTwoRayMin = (size_t)1 << 20;  // two-ray tree-force kernel from this many rays on
 int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int precision, cudaStream_t s,
                        const unsigned long long *d_counts) {
@@ -1111,20 +1209,25 @@ int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int prec
       a.tree_px = ph->theta[0] * ph->Dist;  // LensHalo::getX, as make_halo_dev
       a.tree_py = ph->theta[1] * ph->Dist;
     }
+    const int nb = nblk(n, 128);
     if (d_counts && fld)
-      k_plane_step<GLB_PREC_FP64, true, true><<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step<true, true><<<nb, 128, 0, s>>>(a);
     else if (d_counts)
-      k_plane_step<GLB_PREC_FP64, true><<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step<true, false><<<nb, 128, 0, s>>>(a);
     else if (precision == GLB_PREC_SPLIT && fld)
-      k_plane_step_split<true><<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step_split<true><<<nb, 128, 0, s>>>(a);
     else if (precision == GLB_PREC_SPLIT && ptree)
-      k_plane_step_split_g<<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step_split_g<<<nb, 128, 0, s>>>(a);
     else if (precision == GLB_PREC_SPLIT)
-      k_plane_step_split<<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step_split<<<nb, 128, 0, s>>>(a);
     else if (fld)
-      k_plane_step<GLB_PREC_FP64, false, true><<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step<false, true><<<nb, 128, 0, s>>>(a);
+    else if (l->has_nfw)
+      k_plane_step<false, false><<<nb, 128, 0, s>>>(a);
+    else if (ptree)
+      k_plane_step_f64<true><<<nb, 128, 0, s>>>(a);
     else
-      k_plane_step<GLB_PREC_FP64><<<nblk(n, 128), 128, 0, s>>>(a);
+      k_plane_step_f64<false><<<nb, 128, 0, s>>>(a);
   }
   CKR(cudaGetLastError());
   return 0;
@@ -1374,7 +1477,7 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
   }
   (void)cudaGetLastError();
   if (precision == GLB_PREC_FP64)
-    k_tree_force<<<nblk(n, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
+    k_tree_force_f64<<<nblk(n, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
   else if (precision == GLB_PREC_SPLIT && !t->tree->dev.periodic && n >= kTwoRayMin && t->tree->theta < 0.2)
     k_tree_force_split2<<<nblk((n + 1) / 2, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
   else if (precision == GLB_PREC_SPLIT)

@@ -384,7 +384,8 @@ __global__ void k_pre2slot(const Slot *s, int nslots, int *pre2slot) {
   if (s[i].pre >= 0) pre2slot[s[i].pre] = i;
 }
 
-__global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nodes, GNodeS *snodes) {
+__global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nodes, GNodeS *snodes, TNode *tnodes,
+                             FNode *fnodes) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots) return;
   const Slot &b = s[i];
@@ -409,6 +410,23 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   g.bstart = b.child < 0 ? 0 : b.bstart;
   g.bcount = b.child < 0 ? 0 : b.nbig;
   nodes[b.pre] = g;
+  TNode t;
+  t.cx = g.cx;
+  t.cy = g.cy;
+  // a radius that FP32 squares cannot hold is left to the rays' own tests
+  // (an infinite one, opening angle 0, is still seen as opened by all)
+  const bool fp32 = g.open2 > 1e-30 && g.open2 < 1e30;
+  t.olo = fp32 ? __double2float_rd(g.open2 * (1.0 - 4e-6)) : (g.open2 > 1.0 ? 1e30f : 0.f);
+  t.ohi = fp32 ? __double2float_ru(g.open2 * (1.0 + 4e-6)) : nanf("");
+  t.skip = g.skip;
+  t.info = g.leaf ? 1 : (g.bcount > 0 ? 2 : 0);
+  tnodes[b.pre] = t;
+  FNode fn;
+  fn.mpi = g.mass / kPi;
+  fn.q0pi = g.q0 / kPi;
+  fn.q2pi = g.q2 / kPi;
+  fn.pad = 0;
+  fnodes[b.pre] = fn;
   GNodeS f;
   f.cxh = (float)g.cx;
   f.cyh = (float)g.cy;
@@ -673,7 +691,10 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   // ---- node array
   CK(T->nodes.alloc(nnodes));
   CK(T->snodes.alloc(nnodes));
-  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, T->nodes.p, T->snodes.p);
+  CK(T->tnodes.alloc(nnodes));
+  CK(T->fnodes.alloc(nnodes));
+  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, T->nodes.p, T->snodes.p, T->tnodes.p,
+                                                  T->fnodes.p);
   DBuf<int> dbad;
   CK(dbad.alloc(1));
   CK(cudaMemsetAsync(dbad.p, 0, sizeof(int), st));
@@ -715,6 +736,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   T->dev.root_cy = hphi[7];
   T->dev.nodes = T->nodes.p;
   T->dev.snodes = T->snodes.p;
+  T->dev.tnodes = T->tnodes.p;
+  T->dev.fnodes = T->fnodes.p;
   T->dev.parts = T->parts.p;
   T->dev.bigs = T->bigs.p;
   T->dev.prel = T->prel.p;
