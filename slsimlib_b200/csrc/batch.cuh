@@ -62,6 +62,14 @@ int batch_form(const std::vector<glb_lens *> &lenses, int precision) {
     if (l->has_nfw) return GLB_PREC_FP64;
   return kStripForm;
 }
+// The exponential's tables: those of any particle tree in the batch.
+const ExpTab *batch_exptab(const std::vector<glb_lens *> &lenses) {
+  for (const glb_lens *l : lenses)
+    for (const PlaneHost *p : l->planes)
+      for (const glb_halo *h : p->halos)
+        if (h->tree && h->tree->dev.exptab) return h->tree->dev.exptab;
+  return nullptr;
+}
 // The strip form adds the strip walk's: a StripWarp per warp and the
 // exponential's table.
 inline size_t batch_smem_bytes(int block, int form) {
@@ -124,7 +132,7 @@ template <int PREC>
 // dynamic shared memory: batch_smem_bytes(blockDim.x)
 __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
                                                NFWTables tab, const double *xs, const unsigned *outidx,
-                                               double *y, double *A, int *counter) {
+                                               double *y, double *A, int *counter, const ExpTab *exptab) {
   extern __shared__ __align__(16) double bsm[];
   const int lane = threadIdx.x & 31;
   const int B = blockDim.x;
@@ -136,7 +144,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchun
   if constexpr (PREC == kStripForm) {
     W = reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
     etab = reinterpret_cast<ExpTab *>(reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + B / 32);
-    strip_exp_table(*etab);
+    strip_exp_table(*etab, exptab);
     __syncthreads();
   }
   for (;;) {
@@ -291,14 +299,14 @@ int persistent_grid(int block, int form, int *grid) {
 
 int launch_batch(int form, int grid, int block, cudaStream_t s, const Chunk *chunks, int nchunks,
                  const LensDev *lenses, const NFWTables &tab, const double *xs, const unsigned *outidx, double *y,
-                 double *A, int *counter) {
+                 double *A, int *counter, const ExpTab *exptab) {
   const size_t smem = batch_smem_bytes(block, form);
   if (form == GLB_PREC_SPLIT)
-    k_batch<GLB_PREC_SPLIT><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+    k_batch<GLB_PREC_SPLIT><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
   else if (form == kStripForm)
-    k_batch<kStripForm><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+    k_batch<kStripForm><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
   else
-    k_batch<GLB_PREC_FP64><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter);
+    k_batch<GLB_PREC_FP64><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return fail(GLB_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e) + " launching k_batch with block " +
@@ -379,7 +387,7 @@ int batch_enqueue(glb_batch *b) {
   (void)cudaGetLastError();  // launch errors below are this launch's own
   CKR(cudaMemsetAsync(b->counter.p, 0, sizeof(int), b->stream));
   return launch_batch(b->form, b->grid, b->block, b->stream, b->d_chunks.p, b->nchunks, b->d_lenses.p, b->tab, nullptr,
-                      nullptr, b->y.p, b->A.p, b->counter.p);
+                      nullptr, b->y.p, b->A.p, b->counter.p, batch_exptab(b->lenses));
 }
 }  // namespace
 
@@ -796,7 +804,7 @@ int launch_slot(glb_server *S, Slot &sl) {
   CKR(cudaMemsetAsync(counter, 0, sizeof(int), s));
   if (!C.empty()) {
     if (int rc = launch_batch(S->form, S->grid, 128, s, dch, (int)C.size(), S->d_lenses.p, S->tab, dxs, perm, dy, dA,
-                              counter))
+                              counter, batch_exptab(S->models)))
       return rc;
   }
   // large requests: the lens path's per-plane kernels over the request's rays

@@ -61,6 +61,8 @@ struct Tree {
   DBuf<GNodeS> snodes;
   DBuf<TNode> tnodes;
   DBuf<FNode> fnodes;
+  DBuf<int> cutanc;
+  DBuf<ExpTab> exptab;
   DBuf<float4> parts;
   DBuf<float4> prel;
   DBuf<float4> bigs;

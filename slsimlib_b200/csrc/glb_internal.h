@@ -60,16 +60,26 @@ struct __align__(16) GNodeS {
 struct __align__(16) TNode {
   double cx, cy;   // centre
   float olo, ohi;  // open2 less and plus the classification's margin
-  int skip;
-  int info;        // 1: leaf, 2: internal with softened particles, 0: neither
+  int skip;        // a leaf: its first particle
+  int info;        // a leaf: minus its particle count; 1: internal with softened particles; 0: other
 };
 struct __align__(16) FNode {
   double mpi, q0pi, q2pi, pad;
 };
 
+// Shared walks (several warps per 32 rays) start at multiples of kCutStep nodes.
+constexpr int kCutStep = 16;
+
+// Tables of the strip walk's exponential: exp(-j/1024) and exp(-m).
+struct ExpTab {
+  double lo[1024], hi[704];
+};
+
 struct TreeDev {
   const TNode *tnodes;
   const FNode *fnodes;
+  const int *cutanc;     // kMaxDepth per cut: the ancestors of its node, outermost first, -1 beyond
+  const ExpTab *exptab;
   const GNode *nodes;
   const GNodeS *snodes;
   const float4 *parts;  // sorted particles {x, y, mass, size}

@@ -184,6 +184,7 @@ struct LensWS {
   DBuf<char> sort_tmp;
   DBuf<unsigned long long> bbox;
   DBuf<unsigned char> status;  // per-ray status staging
+  DBuf<char> parts;         // scratch of shared walks
   size_t ws_n = 0;
   float last_kernel_ms = 0, last_total_ms = 0;
   bool timed = false;
@@ -415,18 +416,21 @@ __global__ void k_grid(size_t N1d, double c0, double c1, double range, double *x
 template <int PREC, bool COUNT = false, bool SKIPNEAR = false, bool MERGE = true>
 __device__ __forceinline__ void particle_halo_acc(const TreeDev &T, double rx, double ry, bool valid, double *acc,
                                                   WalkCount *wc = nullptr) {
-  const int im = T.periodic ? 1 : 0;
-  // force2D_recur with a periodic buffer: nine shifted copies (quadTree.h:944-974)
-  for (int i = -im; i <= im; ++i)
-    for (int j = -im; j <= im; ++j) {
-      const double x = im ? rx + i * T.period_x : rx, y = im ? ry + j * T.period_y : ry;
-      if (PREC == GLB_PREC_FP64)
-        walk_f64<COUNT>(T, x, y, valid, acc, wc);
-      else if (PREC == GLB_PREC_FP32)
-        walk_split<true>(T, x, y, valid, acc);
-      else
-        walk_split<false, SKIPNEAR, MERGE>(T, x, y, valid, acc);
-    }
+  auto walk = [&](double x, double y) {
+    if (PREC == GLB_PREC_FP64)
+      walk_f64<COUNT>(T, x, y, valid, acc, wc);
+    else if (PREC == GLB_PREC_FP32)
+      walk_split<true>(T, x, y, valid, acc);
+    else
+      walk_split<false, SKIPNEAR, MERGE>(T, x, y, valid, acc);
+  };
+  if (T.periodic) {
+    // force2D_recur with a periodic buffer: nine shifted copies (quadTree.h:944-974)
+    for (int i = -1; i < 2; ++i)
+      for (int j = -1; j < 2; ++j) walk(rx + i * T.period_x, ry + j * T.period_y);
+  } else {
+    walk(rx, ry);
+  }
 }
 
 // The shared memory of a block's strip walks (walk_strip.cuh).
@@ -483,6 +487,7 @@ struct StepArgs {
   // operands rather than per-thread registers.
   TreeDev tree;
   double tree_px, tree_py;
+  const ExpTab *exptab;  // any tree's (all hold the same values)
 };
 
 // The recursion of include/lens.h:1003-1066 for ray slot k once the plane's
@@ -665,7 +670,7 @@ __global__ void __launch_bounds__(128, 5) k_plane_step_f64(const __grid_constant
   __shared__ StripBlock<128> S;
   __shared__ double sacc[5 * 128];
   const int t = threadIdx.x;
-  strip_exp_table(S.tab);
+  strip_exp_table(S.tab, a.exptab);
   __syncthreads();
   const size_t k = blockIdx.x * (size_t)blockDim.x + t;
   const bool inrange = k < a.n;
@@ -712,6 +717,138 @@ __global__ void __launch_bounds__(128, 5) k_plane_step_f64(const __grid_constant
   }
   if (valid) recursion_step(a, k, al0, al1, kap, g0, g1);
 }
+// Shared walks: calls of too few rays to fill the GPU with one warp per 32 rays
+// split every walk over warps that each take a range of the tree's nodes
+// (walk_strip_part); a second kernel adds the parts of a ray in node order.
+// Warps take (part, group of 32 rays) items from a counter; a part that no ray
+// of the group enters is only flagged.
+struct PartArgs {
+  const double *px, *py;  // positions px[k * stride] * D - ox, py[k * stride] * D - oy
+  size_t stride;
+  double D, ox, oy;
+  const int *jmax_ray;    // per-ray source planes (or null), as StepArgs
+  int j, jmax;
+  size_t n;
+  int nparts, len;        // parts of `len` nodes
+  int *counter;           // 0 at the launch
+  unsigned char *used;    // [group][part]: the part has terms
+  double *out;            // [part][5, or 6 with PHI][n]
+};
+
+template <bool PHI>
+__global__ void __launch_bounds__(128, 5) k_strip_parts(const __grid_constant__ TreeDev T,
+                                                       const __grid_constant__ PartArgs a) {
+  __shared__ StripBlock<128> S;
+  const int lane = threadIdx.x & 31, ngroups = (int)((a.n + 31) / 32), nitems = ngroups * a.nparts;
+  strip_exp_table(S.tab, T.exptab);
+  __syncthreads();
+  for (;;) {
+    int item = 0;
+    if (lane == 0) item = atomicAdd(a.counter, 1);
+    item = __shfl_sync(kFull, item, 0);
+    if (item >= nitems) break;
+    const int part = item / ngroups, group = item - part * ngroups;
+    const size_t k = (size_t)group * 32 + lane;
+    const bool inrange = k < a.n;
+    const bool valid = inrange && a.j < ((a.jmax_ray && inrange) ? a.jmax_ray[k] : a.jmax);
+    bool used = false;
+    if (__any_sync(kFull, valid)) {
+      const double rx = valid ? __dmul_rn(a.px[k * a.stride], a.D) - a.ox : 0.0;
+      const double ry = valid ? __dmul_rn(a.py[k * a.stride], a.D) - a.oy : 0.0;
+      const int s0 = part * a.len, end = min(s0 + a.len, T.nnodes);
+      StripAcc L;
+      used = walk_strip_part<PHI>(T, rx, ry, valid, S.warp[threadIdx.x >> 5], S.tab, s0, end, L);
+      if (used && valid) {
+        double *o = a.out + (size_t)part * (PHI ? 6 : 5) * a.n + k;
+        o[0] = L.a0;
+        o[a.n] = L.a1;
+        o[2 * a.n] = L.k;
+        o[3 * a.n] = L.g0;
+        o[4 * a.n] = 2.0 * L.g1;
+        if (PHI) o[5 * a.n] = L.p;
+      }
+    }
+    if (lane == 0) a.used[(size_t)group * a.nparts + part] = used ? 1 : 0;
+  }
+}
+
+// The sums over the parts of ray k: threads (k, row) each take every
+// kSumRows-th run of parts in order, then the row sums are added in order
+// (in row 0).  A warp reads the used flags of a run at once, so that the loads
+// of the parts in use are in flight together.
+constexpr int kSumRows = 16;
+template <int C>
+__device__ __forceinline__ void sum_parts(const double *part, const unsigned char *used, int nparts, size_t n, size_t k,
+                                          bool valid, double *sum) {
+  __shared__ double rows[kSumRows][C][32];
+  double v[C];
+  for (int c = 0; c < C; ++c) v[c] = 0.0;
+  const unsigned char *u = used + (size_t)blockIdx.x * nparts;
+  const size_t kk = valid ? k : n - 1;
+  const int run = min(32, (nparts + kSumRows - 1) / kSumRows);
+  for (int p0 = run * threadIdx.y; p0 < nparts; p0 += run * kSumRows) {
+    const int p = p0 + threadIdx.x;
+    unsigned m = __ballot_sync(kFull, (int)threadIdx.x < run && p < nparts && u[min(p, nparts - 1)]);
+    while (m) {
+      double w[4][C];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int b = m ? __ffs(m) - 1 : -1;
+        m &= m - 1;
+#pragma unroll
+        for (int c = 0; c < C; ++c) w[i][c] = b >= 0 ? part[((size_t)(p0 + b) * C + c) * n + kk] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] += w[i][c];
+    }
+  }
+  for (int c = 0; c < C; ++c) rows[threadIdx.y][c][threadIdx.x] = v[c];
+  __syncthreads();
+  if (threadIdx.y == 0)
+    for (int c = 0; c < C; ++c) {
+      double t = 0;
+      for (int r = 0; r < kSumRows; ++r) t += rows[r][c][threadIdx.x];
+      sum[c] = t;
+    }
+}
+
+// The plane step of shared walks: the particle halo's parts, the plane's
+// analytic halos and the recursion.
+__global__ void __launch_bounds__(32 * kSumRows) k_plane_parts_end(const __grid_constant__ StepArgs a,
+                                                                  const double *part, const unsigned char *used,
+                                                                  int nparts) {
+  const size_t k = blockIdx.x * (size_t)32 + threadIdx.x;
+  const bool inrange = k < a.n;
+  const bool valid = inrange && a.j < ((a.jmax_ray && inrange) ? a.jmax_ray[k] : a.jmax);
+  double acc[5];
+  sum_parts<5>(part, used, nparts, a.n, k, valid, acc);
+  if (threadIdx.y != 0 || !valid) return;
+  if (a.tree.inv_area != 0.0) acc[2] -= a.tree.inv_area * a.tree.root_mass;
+  const PlaneDev P = a.planes[a.j];
+  const double xx0 = __dmul_rn(a.st[k], P.Dphys), xx1 = __dmul_rn(a.st[a.n + k], P.Dphys);
+  double al0 = 0, al1 = 0, kap = 0, g0 = 0, g1 = 0;
+  for (int h = 0; h < P.nhalo; ++h) {
+    const HaloDev *H = a.halos + P.halo0 + h;
+    if (H->kind == HALO_PARTICLES) {
+      al0 += acc[0];
+      al1 += acc[1];
+      kap += acc[2];
+      g0 += acc[3];
+      g1 += acc[4];
+    } else {
+      const Force5 f = analytic_halo(H, &a.tab, xx0 - H->px, xx1 - H->py);
+      al0 -= f.a0;
+      al1 -= f.a1;
+      kap += f.k;
+      g0 += f.g0;
+      g1 += f.g1;
+    }
+  }
+  recursion_step(a, k, al0, al1, kap, g0, g1);
+}
+
 // Split-form plane step with the block-level group walk (walk_group.cuh) for
 // a plane holding exactly one particle halo (its tree in a.tree, a kernel
 // parameter) and any number of analytic halos: one ray per thread, 128
@@ -803,16 +940,12 @@ __global__ void __launch_bounds__(128, 8) k_plane_step_split(const __grid_consta
   plane_step<GLB_PREC_SPLIT, false, FIELD>(a);
 }
 
-// force2D_recur / force_halo at arbitrary positions (walk-level API, with phi).
+// force_halo of analytic haloes and field planes at arbitrary positions, with phi.
 // subtract: LensHalo::force_halo's subtract_point = true with `screening`
 // (analytic haloes; particle trees and field planes take no such argument).
 __global__ void __launch_bounds__(128) k_halo_force(HaloDev H, NFWTables tab, size_t n, const double *x,
                                                     double *out, int subtract = 0, double screening = 1.0) {
-  __shared__ StripBlock<128> S;
-  const int t = threadIdx.x;
-  strip_exp_table(S.tab);
-  __syncthreads();
-  const size_t k = blockIdx.x * (size_t)blockDim.x + t;
+  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const bool valid = k < n;
   if (!__any_sync(kFull, valid)) return;
   double x0 = 0, x1 = 0;
@@ -821,9 +954,7 @@ __global__ void __launch_bounds__(128) k_halo_force(HaloDev H, NFWTables tab, si
     x1 = x[2 * k + 1];
   }
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  if (H.kind == HALO_PARTICLES) {
-    particle_halo_f64<true>(H.tree, x0, x1, valid, S.warp[t >> 5], S.tab, acc, 1);
-  } else if (H.kind == HALO_FIELD) {
+  if (H.kind == HALO_FIELD) {
     field_plane_acc<true>(H.htree, tab, x0, x1, valid, acc);
   } else if (valid && subtract) {
     if (H.kind == HALO_NFW) {
@@ -864,7 +995,7 @@ __global__ void __launch_bounds__(128, 5) k_tree_force_f64(const __grid_constant
                                                           const double *x, double *out) {
   __shared__ StripBlock<128> S;
   const int t = threadIdx.x;
-  strip_exp_table(S.tab);
+  strip_exp_table(S.tab, T.exptab);
   __syncthreads();
   const size_t k = blockIdx.x * (size_t)blockDim.x + t;
   const bool valid = k < n;
@@ -884,6 +1015,62 @@ template <int PREC>
 __global__ void __launch_bounds__(128, 6) k_tree_force_lo(const __grid_constant__ TreeDev T, size_t n,
                                                           const double *x, double *out) {
   tree_force<PREC>(T, n, x, out);
+}
+
+// force2D_recur with the potential for host callers: rays in Morton order
+// (positions px, py), results to the caller's order.
+struct ForceOut {
+  double *alpha, *kappa, *gamma, *phi;  // 2n, n, 3n, n
+  __device__ __forceinline__ void put(size_t i, const double *acc) const {
+    alpha[2 * i] = acc[0];
+    alpha[2 * i + 1] = acc[1];
+    kappa[i] = acc[2];
+    gamma[3 * i] = acc[3];
+    gamma[3 * i + 1] = acc[4];
+    gamma[3 * i + 2] = 0.0;
+    phi[i] = acc[5];
+  }
+};
+__global__ void k_gather_xy(const double *x, const unsigned *perm, size_t n, double *px, double *py) {
+  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const size_t i = perm[k];
+  px[k] = x[2 * i];
+  py[k] = x[2 * i + 1];
+}
+__global__ void __launch_bounds__(128, 4) k_tree_force_phi(const __grid_constant__ TreeDev T, size_t n, const double *px,
+                                                          const double *py, const unsigned *perm, ForceOut out) {
+  __shared__ StripBlock<128> S;
+  const int t = threadIdx.x;
+  strip_exp_table(S.tab, T.exptab);
+  __syncthreads();
+  const size_t k = blockIdx.x * (size_t)blockDim.x + t;
+  const bool valid = k < n;
+  if (!__any_sync(kFull, valid)) return;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  particle_halo_f64<true>(T, valid ? px[k] : 0.0, valid ? py[k] : 0.0, valid, S.warp[t >> 5], S.tab, acc, 1);
+  if (valid) out.put(perm[k], acc);
+}
+__global__ void __launch_bounds__(32 * kSumRows) k_force_parts_end(const __grid_constant__ TreeDev T, size_t n,
+                                                                  const double *part, const unsigned char *used,
+                                                                  int nparts, const unsigned *perm, ForceOut out) {
+  const size_t k = blockIdx.x * (size_t)32 + threadIdx.x;
+  double acc[6];
+  sum_parts<6>(part, used, nparts, n, k, k < n, acc);
+  if (threadIdx.y != 0 || k >= n) return;
+  if (T.inv_area != 0.0) acc[2] -= T.inv_area * T.root_mass;
+  out.put(perm[k], acc);
+}
+
+__global__ void __launch_bounds__(32 * kSumRows) k_force5_parts_end(const __grid_constant__ TreeDev T, size_t n,
+                                                                   const double *part, const unsigned char *used,
+                                                                   int nparts, double *out) {
+  const size_t k = blockIdx.x * (size_t)32 + threadIdx.x;
+  double acc[5];
+  sum_parts<5>(part, used, nparts, n, k, k < n, acc);
+  if (threadIdx.y != 0 || k >= n) return;
+  if (T.inv_area != 0.0) acc[2] -= T.inv_area * T.root_mass;
+  for (int c = 0; c < 5; ++c) out[5 * k + c] = acc[c];
 }
 
 // The split form with two rays per thread (rays 2g and 2g + 1; a warp walks
@@ -1179,6 +1366,75 @@ int ensure_ws(LensWS *w, size_t n, bool per_ray) {
   return 0;
 }
 
+// How a walk of n rays over a tree of nnodes is shared: parts per walk (1: one
+// warp walks alone) and their length.  About kPartItems (part, group) items in
+// all, for 2,960 resident warps (20 an SM), so that uneven parts balance.
+constexpr size_t kPartItems = 65536;
+int strip_parts(size_t n, size_t max_rays, int nnodes, int *len) {
+  *len = nnodes;
+  if (n == 0 || n >= max_rays || nnodes == 0) return 1;
+  const size_t groups = (n + 31) / 32, cuts = ((size_t)nnodes + kCutStep - 1) / kCutStep;
+  const size_t want = std::min((kPartItems + groups - 1) / groups, cuts);
+  const size_t per = (cuts + want - 1) / want;
+  *len = (int)(per * kCutStep);
+  return (int)((cuts + per - 1) / per);
+}
+// Plane steps share walks below this many rays; from here on a call has a warp
+// for every slot of the GPU by itself.
+constexpr size_t kPlanePartsMax = (size_t)1 << 16;
+// Tree forces likewise (one walk per ray, so that a last, partly filled wave
+// weighs more than in a lens's planes).
+constexpr size_t kForcePartsMax = (size_t)1 << 18;
+
+// The particle halo of a plane that holds exactly one and no field plane
+// (periodic trees, which LensHaloParticles never builds, are left to the
+// general kernels), or null.
+const glb_halo *single_tree(const glb_lens *l, int j) {
+  const glb_halo *ph = nullptr;
+  for (const glb_halo *h : l->planes[j]->halos)
+    if (h->kind == HALO_PARTICLES) {
+      if (ph) return nullptr;
+      ph = h;
+    }
+  return ph && ph->tree && !l->plane_field[j] && !ph->tree->dev.periodic ? ph : nullptr;
+}
+
+// The scratch of shared walks: [sums of the parts][counters][used flags].
+constexpr int kPartCounters = 256;  // launches between two clearings of the counters
+size_t parts_bytes(size_t n, int parts, int comps) {
+  return (size_t)parts * comps * n * sizeof(double) + kPartCounters * sizeof(int) + (size_t)parts * ((n + 31) / 32);
+}
+// Points p at scratch for launch number i of a pass (its counter cleared by
+// clear_part_counters).
+void set_part_scratch(PartArgs &p, char *scratch, size_t sums, int i) {
+  p.out = (double *)scratch;
+  p.counter = (int *)(scratch + sums) + i % kPartCounters;
+  p.used = (unsigned char *)((int *)(scratch + sums) + kPartCounters);
+}
+template <bool PHI>
+int launch_parts(const TreeDev &T, const PartArgs &p, cudaStream_t s) {
+  int dev = 0, sms = 0;
+  CKR(cudaGetDevice(&dev));
+  CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const size_t items = ((p.n + 31) / 32) * p.nparts;
+  k_strip_parts<PHI><<<(int)std::min<size_t>(5 * sms, (items + 3) / 4), 128, 0, s>>>(T, p);
+  return 0;
+}
+
+// Bytes of the sums that the shared walks of n rays through l take (0: no
+// walk of the call is shared).
+size_t parts_sums(const glb_lens *l, size_t n, int precision) {
+  size_t m = 0;
+  if (precision != GLB_PREC_FP64 || l->has_nfw) return 0;
+  for (size_t j = 0; j < l->planes.size(); ++j)
+    if (const glb_halo *ph = single_tree(l, (int)j)) {
+      int len;
+      const int parts = strip_parts(n, kPlanePartsMax, ph->tree->dev.nnodes, &len);
+      if (parts > 1) m = std::max(m, (size_t)parts * 5 * n * sizeof(double));
+    }
+  return m;
+}
+
 // One launch per plane, in order.  Split-form planes that hold exactly one
 // particle halo and no field plane run the group walk (k_plane_step_split_g,
 // the tree in the kernel parameters); planes with a field plane use the FIELD
@@ -1187,27 +1443,47 @@ int ensure_ws(LensWS *w, size_t n, bool per_ray) {
 // bin cancel up to 1e9-fold (nfw_g, nfw_g2), so a ray that meets a halo's
 // centre carries the last bit of its position into the ninth digit of A, and
 // those lenses keep the walk whose last bits are the reference's operations.
+// Small FP64 calls share their walks (strip_parts) where the caller has scratch
+// for them (parts_sums).
 constexpr size_t kTwoRayMin = (size_t)1 << 20;  // two-ray tree-force kernel from this many rays on
 int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int precision, cudaStream_t s,
-                       const unsigned long long *d_counts) {
+                       const unsigned long long *d_counts, char *scratch = nullptr, size_t sums = 0) {
   const size_t n = a.n;
   for (int j = 0; j < jmax_launch; ++j) {
     a.j = j;
     const bool fld = l->plane_field[j] != 0;
-    int npart = 0;
-    const glb_halo *ph = nullptr;
-    for (const glb_halo *h : l->planes[j]->halos)
-      if (h->kind == HALO_PARTICLES) {
-        ++npart;
-        ph = h;
-      }
-    const bool ptree = npart == 1 && ph->tree && !fld && !ph->tree->dev.periodic;  // the group walk has no periodic images
+    const glb_halo *ph = single_tree(l, j);
+    const bool ptree = ph != nullptr;
     memset(&a.tree, 0, sizeof(a.tree));
     a.tree_px = a.tree_py = 0;
+    a.exptab = nullptr;
+    for (const glb_halo *h : l->planes[j]->halos)
+      if (h->tree && h->tree->dev.exptab) a.exptab = h->tree->dev.exptab;
     if (ptree) {
       a.tree = ph->tree->dev;
       a.tree_px = ph->theta[0] * ph->Dist;  // LensHalo::getX, as make_halo_dev
       a.tree_py = ph->theta[1] * ph->Dist;
+    }
+    if (scratch && j % kPartCounters == 0) CKR(cudaMemsetAsync(scratch + sums, 0, kPartCounters * sizeof(int), s));
+    if (scratch && !d_counts && precision == GLB_PREC_FP64 && !l->has_nfw && ptree) {
+      PartArgs p;
+      p.nparts = strip_parts(n, kPlanePartsMax, a.tree.nnodes, &p.len);
+      if (p.nparts > 1) {
+        p.px = a.st;
+        p.py = a.st + n;
+        p.stride = 1;
+        p.D = l->Dl[j] / (1 + l->plane_z[j]);  // PlaneDev::Dphys
+        p.ox = a.tree_px;
+        p.oy = a.tree_py;
+        p.jmax_ray = a.jmax_ray;
+        p.j = j;
+        p.jmax = a.jmax;
+        p.n = n;
+        set_part_scratch(p, scratch, sums, j);
+        if (int rc = launch_parts<false>(a.tree, p, s)) return rc;
+        k_plane_parts_end<<<nblk(n, 32), dim3(32, kSumRows), 0, s>>>(a, p.out, p.used, p.nparts);
+        continue;
+      }
     }
     const int nb = nblk(n, 128);
     if (d_counts && fld)
@@ -1269,6 +1545,12 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
   }
   if (int rc = upload_lens(l)) return rc;
   if (int rc = ensure_ws(w, n, zs != nullptr)) return rc;
+  // shared walks: calls below kPlanePartsMax rays, which run in one slab
+  const size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
+  if (psums) {
+    const size_t pb = psums + parts_bytes(n, 0, 0) + psums / (5 * sizeof(double)) + 256;  // sums, counters, flags
+    if (w->parts.n < pb) CKR(w->parts.alloc(pb));
+  }
   CKR(cudaStreamWaitEvent(s, w->done, 0));
   CKR(cudaEventRecord(w->ev[0], s));
   // spatial ordering of the rays along a Morton curve
@@ -1337,7 +1619,8 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
     ai.n = mi;
     ai.jmax_ray = zs ? w->jmax_ray.p + o : nullptr;
     ai.src_ray = zs ? w->src_ray.p + 2 * o : nullptr;
-    if (int rc = launch_plane_steps(l, ai, jmax_launch, precision, si, d_counts)) return rc;
+    if (int rc = launch_plane_steps(l, ai, jmax_launch, precision, si, d_counts, psums ? w->parts.p : nullptr, psums))
+      return rc;
     k_finish<<<nblk(mi, 256), 256, 0, si>>>(ai.st, w->perm.p + o, mi, y, A, status, skip);
     if (i > 0) {
       CKR(cudaEventRecord(w->join[i - 1], si));
@@ -1373,6 +1656,13 @@ struct glb_tree {
   std::unique_ptr<Tree> tree;
   int device = 0;
   cudaStream_t stream = nullptr;
+  std::mutex mu;     // guards ws
+  DBuf<char> ws;     // force2D_recur's device workspace
+  // scratch of the device-array call's shared walks; calls that use it are
+  // ordered on the GPU by dev_done, whatever their streams
+  std::mutex dev_mu;
+  DBuf<char> dev_ws;
+  cudaEvent_t dev_done = nullptr;
 };
 
 int glb_tree_create(const glb_particle *particles, size_t n, float mass_fixed, float size_fixed, double inv_area,
@@ -1407,16 +1697,89 @@ int glb_tree_destroy(glb_tree *t) {
   if (!t) return 0;
   cudaSetDevice(t->device);
   t->tree.reset();
+  t->ws.release();
+  t->dev_ws.release();
+  if (t->dev_done) cudaEventDestroy(t->dev_done);
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;
   return 0;
 }
 
+// A particle tree's forces and potential at host positions: rays sorted along
+// a Morton curve (neighbouring rays of a warp share the walk's decisions; each
+// ray's result is its own), walks shared by several warps in small calls.
+// ws: the caller's workspace, grown as needed.
+static int force_particles(const TreeDev &T, cudaStream_t s, DBuf<char> &ws, size_t n, const double *xcm,
+                           double *alpha, double *kappa, double *gamma, double *phi) {
+  PartArgs p;
+  p.nparts = T.periodic ? 1 : strip_parts(n, kForcePartsMax, T.nnodes, &p.len);
+  size_t tb = 0;
+  CKR(cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned *)nullptr, (unsigned *)nullptr, (unsigned *)nullptr,
+                                      (unsigned *)nullptr, (int)n, 0, 32, s));
+  auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t o_x = 0, o_xy = o_x + al(16 * n), o_out = o_xy + al(16 * n), o_k = o_out + al(56 * n);
+  const size_t o_perm = o_k + al(8 * n), o_bb = o_perm + al(8 * n), o_tmp = o_bb + 256, o_part = o_tmp + al(tb);
+  const size_t sums = (size_t)p.nparts * 6 * n * sizeof(double);
+  const size_t need = o_part + (p.nparts > 1 ? parts_bytes(n, p.nparts, 6) : 0);
+  if (ws.n < need) CKR(ws.alloc(need));
+  char *m = ws.p;
+  double *dx = (double *)(m + o_x), *px = (double *)(m + o_xy), *py = px + n, *out = (double *)(m + o_out);
+  unsigned *keys = (unsigned *)(m + o_k), *perm0 = (unsigned *)(m + o_perm), *perm = perm0 + n;
+  CKR(cudaMemcpyAsync(dx, xcm, 2 * n * sizeof(double), cudaMemcpyHostToDevice, s));
+  if (n >= 64) {
+    static const unsigned long long init[4] = {~0ull, ~0ull, 0ull, 0ull};
+    unsigned long long *bb = (unsigned long long *)(m + o_bb);
+    CKR(cudaMemcpyAsync(bb, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_ray_bbox<<<std::min(nblk(n, 256), 1184), 256, 0, s>>>(dx, n, bb);
+    k_ray_morton<<<nblk(n, 256), 256, 0, s>>>(dx, n, bb, keys, perm0);
+    CKR(cub::DeviceRadixSort::SortPairs(m + o_tmp, tb, keys, keys + n, perm0, perm, (int)n, 0, 32, s));
+  } else {
+    k_identity<<<nblk(n, 256), 256, 0, s>>>(perm, n);
+  }
+  k_gather_xy<<<nblk(n, 256), 256, 0, s>>>(dx, perm, n, px, py);
+  const ForceOut fo{out, out + 2 * n, out + 3 * n, out + 6 * n};
+  if (p.nparts > 1) {
+    p.px = px;
+    p.py = py;
+    p.stride = 1;
+    p.D = 1.0;
+    p.ox = p.oy = 0.0;
+    p.jmax_ray = nullptr;
+    p.j = 0;
+    p.jmax = 1;
+    p.n = n;
+    set_part_scratch(p, m + o_part, sums, 0);
+    CKR(cudaMemsetAsync(p.counter, 0, sizeof(int), s));
+    if (int rc = launch_parts<true>(T, p, s)) return rc;
+    k_force_parts_end<<<nblk(n, 32), dim3(32, kSumRows), 0, s>>>(T, n, p.out, p.used, p.nparts, perm, fo);
+  } else {
+    k_tree_force_phi<<<nblk(n, 128), 128, 0, s>>>(T, n, px, py, perm, fo);
+  }
+  CKR(cudaGetLastError());
+  if (alpha) CKR(cudaMemcpyAsync(alpha, fo.alpha, 2 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if (kappa) CKR(cudaMemcpyAsync(kappa, fo.kappa, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if (gamma) CKR(cudaMemcpyAsync(gamma, fo.gamma, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if (phi) CKR(cudaMemcpyAsync(phi, fo.phi, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  CKR(cudaStreamSynchronize(s));
+  return 0;
+}
+
 static int force_generic(const HaloDev &H, int device, cudaStream_t s, size_t n, const double *xcm, double *alpha,
-                         double *kappa, double *gamma, double *phi, int subtract = 0, double screening = 1.0) {
+                         double *kappa, double *gamma, double *phi, int subtract = 0, double screening = 1.0,
+                         DBuf<char> *ws = nullptr) {
   if (n == 0) return 0;
   if (!xcm) return fail(GLB_ERR_ARG, "null positions");
   if (int rc = set_dev(device)) return rc;
+  if (H.kind == HALO_PARTICLES) {
+    DBuf<char> local;
+    constexpr size_t kChunk = (size_t)1 << 24;  // bounds the workspace
+    for (size_t o = 0; o < n; o += kChunk)
+      if (int rc = force_particles(H.tree, s, ws ? *ws : local, std::min(kChunk, n - o), xcm + 2 * o,
+                                   alpha ? alpha + 2 * o : nullptr, kappa ? kappa + o : nullptr,
+                                   gamma ? gamma + 3 * o : nullptr, phi ? phi + o : nullptr))
+        return rc;
+    return 0;
+  }
   NFWTables tab{};
   if (H.kind == HALO_NFW || H.kind == HALO_FIELD)
     if (int rc = device_nfw_tables(tab)) return rc;
@@ -1461,7 +1824,12 @@ int glb_tree_force2D_recur(glb_tree *t, size_t n, const double *rays, double *al
     }
     return 0;
   }
-  return force_generic(H, t->device, t->stream, n, rays, alpha, kappa, gamma, phi);
+  // one caller at a time uses the tree's workspace; others take their own
+  std::unique_lock<std::mutex> lk(t->mu, std::try_to_lock);
+  const int rc = force_generic(H, t->device, t->stream, n, rays, alpha, kappa, gamma, phi, 0, 1.0,
+                               lk.owns_lock() ? &t->ws : nullptr);
+  if (lk.owns_lock() && t->ws.n > ((size_t)64 << 20)) t->ws.release();  // a large call's is given back
+  return rc;
 }
 
 int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double *out_dev, int precision,
@@ -1476,6 +1844,36 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
     return 0;
   }
   (void)cudaGetLastError();
+  if (precision == GLB_PREC_FP64 && !t->tree->dev.periodic) {
+    PartArgs p;
+    p.nparts = strip_parts(n, kPlanePartsMax, t->tree->dev.nnodes, &p.len);
+    // a stream in capture cannot wait for earlier calls' use of the scratch
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (p.nparts > 1) CKR(cudaStreamIsCapturing(s, &cap));
+    if (p.nparts > 1 && cap == cudaStreamCaptureStatusNone) {
+      std::lock_guard<std::mutex> lk(t->dev_mu);
+      const size_t need = parts_bytes(n, p.nparts, 5);
+      if (t->dev_ws.n < need) CKR(t->dev_ws.alloc(need));
+      if (!t->dev_done) CKR(cudaEventCreateWithFlags(&t->dev_done, cudaEventDisableTiming));
+      CKR(cudaStreamWaitEvent(s, t->dev_done, 0));
+      p.px = rays_dev;
+      p.py = rays_dev + 1;
+      p.stride = 2;
+      p.D = 1.0;
+      p.ox = p.oy = 0.0;
+      p.jmax_ray = nullptr;
+      p.j = 0;
+      p.jmax = 1;
+      p.n = n;
+      set_part_scratch(p, t->dev_ws.p, (size_t)p.nparts * 5 * n * sizeof(double), 0);
+      CKR(cudaMemsetAsync(p.counter, 0, sizeof(int), s));
+      if (int rc = launch_parts<false>(t->tree->dev, p, s)) return rc;
+      k_force5_parts_end<<<nblk(n, 32), dim3(32, kSumRows), 0, s>>>(t->tree->dev, n, p.out, p.used, p.nparts, out_dev);
+      CKR(cudaEventRecord(t->dev_done, s));
+      CKR(cudaGetLastError());
+      return 0;
+    }
+  }
   if (precision == GLB_PREC_FP64)
     k_tree_force_f64<<<nblk(n, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
   else if (precision == GLB_PREC_SPLIT && !t->tree->dev.periodic && n >= kTwoRayMin && t->tree->theta < 0.2)

@@ -418,8 +418,8 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   const bool fp32 = g.open2 > 1e-30 && g.open2 < 1e30;
   t.olo = fp32 ? __double2float_rd(g.open2 * (1.0 - 4e-6)) : (g.open2 > 1.0 ? 1e30f : 0.f);
   t.ohi = fp32 ? __double2float_ru(g.open2 * (1.0 + 4e-6)) : nanf("");
-  t.skip = g.skip;
-  t.info = g.leaf ? 1 : (g.bcount > 0 ? 2 : 0);
+  t.skip = g.leaf ? g.pstart : g.skip;
+  t.info = g.leaf ? -g.pcount : (g.bcount > 0 ? 1 : 0);
   tnodes[b.pre] = t;
   FNode fn;
   fn.mpi = g.mass / kPi;
@@ -445,6 +445,26 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   f.start = g.leaf ? g.pstart : g.bstart;
   f.count = g.leaf ? g.pcount : g.bcount;
   snodes[b.pre] = f;
+}
+
+// The ancestors of every kCutStep-th node, outermost first.
+__global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= ncut) return;
+  const int s = g * kCutStep;
+  int *a = anc + (size_t)kMaxDepth * g, k = 0, node = 0;
+  while (node < s && k < kMaxDepth) {
+    const int skip = t[node].info < 0 ? node + 1 : t[node].skip;
+    if (skip > s) a[k++] = node++;  // the cut lies below it
+    else node = skip;
+  }
+  for (; k < kMaxDepth; ++k) a[k] = -1;
+}
+
+__global__ void k_exp_tables(ExpTab *E) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 1024) E->lo[i] = exp(-(double)i / 1024.0);
+  if (i < 704) E->hi[i] = exp(-(double)i);
 }
 
 __global__ void k_gather_parts(const glb_particle_rec *p, const unsigned *sidx, int n, int multimass,
@@ -695,6 +715,11 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   CK(T->fnodes.alloc(nnodes));
   k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, T->nodes.p, T->snodes.p, T->tnodes.p,
                                                   T->fnodes.p);
+  const int ncut = (nnodes + kCutStep - 1) / kCutStep;
+  CK(T->cutanc.alloc((size_t)ncut * kMaxDepth));
+  CK(T->exptab.alloc(1));
+  k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(T->tnodes.p, ncut, T->cutanc.p);
+  k_exp_tables<<<4, 256, 0, st>>>(T->exptab.p);
   DBuf<int> dbad;
   CK(dbad.alloc(1));
   CK(cudaMemsetAsync(dbad.p, 0, sizeof(int), st));
@@ -738,6 +763,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   T->dev.snodes = T->snodes.p;
   T->dev.tnodes = T->tnodes.p;
   T->dev.fnodes = T->fnodes.p;
+  T->dev.cutanc = T->cutanc.p;
+  T->dev.exptab = T->exptab.p;
   T->dev.parts = T->parts.p;
   T->dev.bigs = T->bigs.p;
   T->dev.prel = T->prel.p;

@@ -64,9 +64,6 @@ __device__ __forceinline__ double strip_rcp(double a) {
 // 2e-11 and the rounding of its constant 6e-7 of it), so that they are
 // immediates; full double constants cost two instructions each per use.  t is
 // held at 700 (by its high word), where exp(-t) is below 1e-304.
-struct ExpTab {
-  double lo[1024], hi[704];
-};
 constexpr double kC3 = -0x1.55555p-3, kC4 = 0x1.55555p-5;
 __device__ __forceinline__ double strip_exp_neg(double t, const ExpTab &E) {
   constexpr double kShift = 6755399441055744.0;  // 1.5 * 2^52
@@ -81,9 +78,12 @@ __device__ __forceinline__ double strip_exp_neg(double t, const ExpTab &E) {
   return __fma_rn(e, __dmul_rn(r, p), e);
 }
 
-__device__ __forceinline__ void strip_exp_table(ExpTab &E) {
-  for (int i = threadIdx.x; i < 1024; i += blockDim.x) E.lo[i] = exp(-(double)i / 1024.0);
-  for (int i = threadIdx.x; i < 704; i += blockDim.x) E.hi[i] = exp(-(double)i);
+// A block's copy of the tables.
+__device__ __forceinline__ void strip_exp_table(ExpTab &E, const ExpTab *src) {
+  if (!src) return;  // no tree with nodes: the tables are not read
+  const double2 *f = reinterpret_cast<const double2 *>(src);
+  double2 *t = reinterpret_cast<double2 *>(&E);
+  for (int i = threadIdx.x; i < (int)(sizeof(ExpTab) / sizeof(double2)); i += blockDim.x) t[i] = __ldg(f + i);
 }
 
 // The tree as a walk reads it, by value: fields of a descriptor in global
@@ -135,23 +135,32 @@ struct StripWalk {
   int lane;
 };
 
+// FP32 keys in the order of their values, for the integer warp reductions.
+__device__ __forceinline__ int f_key(float f) {
+  const int b = __float_as_int(f);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float key_f(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+// The box is that of the rays rounded outwards to FP32 (a warp's rays spread
+// far wider than that); rays that are not finite stay out of it (whatever their
+// nodes' classes, their sums are not finite).
 __device__ __forceinline__ StripWalk strip_begin(double rx, double ry, bool valid) {
   StripWalk w;
   w.rx = rx;
   w.ry = ry;
   w.lane = threadIdx.x & 31;
   w.vmask = __ballot_sync(kFull, valid);
-  double a = valid ? rx : 1e300, b = valid ? rx : -1e300, c = valid ? ry : 1e300, d = valid ? ry : -1e300;
-  for (int o = 16; o > 0; o >>= 1) {
-    a = fmin(a, __shfl_xor_sync(kFull, a, o));
-    b = fmax(b, __shfl_xor_sync(kFull, b, o));
-    c = fmin(c, __shfl_xor_sync(kFull, c, o));
-    d = fmax(d, __shfl_xor_sync(kFull, d, o));
-  }
-  w.bx = 0.5 * (a + b);
-  w.by = 0.5 * (c + d);
-  w.hx = __double2float_ru(fmax(b - w.bx, w.bx - a)) * 1.000001f;
-  w.hy = __double2float_ru(fmax(d - w.by, w.by - c)) * 1.000001f;
+  const bool in = valid && isfinite(rx) && isfinite(ry);
+  constexpr float kBig = 1e30f;
+  const float x0 = key_f(__reduce_min_sync(kFull, f_key(in ? __double2float_rd(rx) : kBig)));
+  const float x1 = key_f(__reduce_max_sync(kFull, f_key(in ? __double2float_ru(rx) : -kBig)));
+  const float y0 = key_f(__reduce_min_sync(kFull, f_key(in ? __double2float_rd(ry) : kBig)));
+  const float y1 = key_f(__reduce_max_sync(kFull, f_key(in ? __double2float_ru(ry) : -kBig)));
+  w.bx = 0.5 * ((double)x0 + (double)x1);
+  w.by = 0.5 * ((double)y0 + (double)y1);
+  w.hx = __double2float_ru(0.5 * ((double)x1 - (double)x0)) * 1.000001f;
+  w.hy = __double2float_ru(0.5 * ((double)y1 - (double)y0)) * 1.000001f;
   return w;
 }
 
@@ -221,10 +230,11 @@ __device__ __forceinline__ void strip_push(const StripWalk &w, StripWarp &W, Str
 // A leaf opened by the rays of `om`: its particles as point masses, with their
 // softening where the leaf applies it (quadTree.h:1017-1077).
 template <bool PHI, bool SCREEN, bool SHEET>
-__device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk &w, StripWarp &W, int node, unsigned om,
-                                           const ExpTab &tab, StripAcc &L) {
+__device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk &w, StripWarp &W, int node, int p0, int n,
+                                           unsigned om, const ExpTab &tab, StripAcc &L) {
+  float4 Q = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (w.lane < n) Q = __ldg(T.parts + p0 + w.lane);  // in flight with the node's row
   const GNode *nd = T.nodes + node;
-  const int p0 = nd->pstart, n = nd->pcount;
   const double width = nd->width;
   const bool mine = om >> w.lane & 1u;
   const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
@@ -238,7 +248,7 @@ __device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk &
     const int m = min(32, n - q0);
     __syncwarp();
     if (w.lane < m) {
-      const float4 Q = __ldg(T.parts + p0 + q0 + w.lane);
+      if (q0) Q = __ldg(T.parts + p0 + q0 + w.lane);
       const double size = (double)Q.w;
       W.part[2 * w.lane] = make_double2((double)Q.x, (double)Q.y);
       // mass / pi, and the squared radius of the softening this leaf applies
@@ -315,7 +325,7 @@ __device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk 
   const bool mine = w.vmask >> w.lane & 1u;
   StripQueue q;
   while (base < end) {
-    const int i = base + w.lane;
+    const int sbase = base, i = base + w.lane;
     const bool in = i < end;
     int skip = 0, info = 0, cls = 3;
     double2 r0 = make_double2(0, 0);
@@ -327,6 +337,8 @@ __device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk 
       info = __float_as_int(o.w);
       cls = strip_class(w, r0.x, r0.y, o.x, o.y);
     }
+    const int pstart = skip;
+    if (info < 0) skip = i + 1;
     // strip positions inside the subtree of an A node before them
     const int span = min(skip - base, 32);
     const unsigned cov =
@@ -408,12 +420,23 @@ __device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk 
         q.masked = false;
       }
       if (node < 0) break;
-      if (inf & 1)
-        strip_leaf<PHI, SCREEN, SHEET>(T, w, W, node, om, tab, L);
+      if (inf < 0)
+        strip_leaf<PHI, SCREEN, SHEET>(T, w, W, node, __shfl_sync(kFull, pstart, node - sbase), -inf, om, tab, L);
       else
         strip_bigs<PHI>(T, w, node, om, L);
     }
   }
+}
+
+template <bool PHI>
+__device__ __forceinline__ void strip_run(const StripTree &T, const StripWalk &w, StripWarp &W, const ExpTab &tab,
+                                          int base, int end, int resume, StripAcc &L) {
+  if (T.pia != 0.0)
+    strip_range<PHI, true, true>(T, w, W, tab, base, end, resume, L);
+  else if (T.s2 != 0.0)
+    strip_range<PHI, true, false>(T, w, W, tab, base, end, resume, L);
+  else
+    strip_range<PHI, false, false>(T, w, W, tab, base, end, resume, L);
 }
 
 // One whole walk for the ray (rx, ry), added to acc[c * A], c = 0..4 (and 5,
@@ -426,13 +449,7 @@ __device__ __forceinline__ void walk_strip(const TreeDev &D, double rx, double r
   const StripTree T(D);
   const StripWalk w = strip_begin(rx, ry, valid);
   StripAcc L;
-  int base = 0, resume = valid ? 0 : 0x7fffffff;
-  if (T.pia != 0.0)
-    strip_range<PHI, true, true>(T, w, W, tab, base, nn, resume, L);
-  else if (T.s2 != 0.0)
-    strip_range<PHI, true, false>(T, w, W, tab, base, nn, resume, L);
-  else
-    strip_range<PHI, false, false>(T, w, W, tab, base, nn, resume, L);
+  strip_run<PHI>(T, w, W, tab, 0, nn, valid ? 0 : 0x7fffffff, L);
   acc[0] += L.a0;
   acc[A] += L.a1;
   acc[2 * A] += L.k;
@@ -440,6 +457,42 @@ __device__ __forceinline__ void walk_strip(const TreeDev &D, double rx, double r
   acc[4 * A] += 2.0 * L.g1;
   if (PHI) acc[5 * A] += L.p;
   if (D.inv_area != 0.0 && valid) acc[2 * A] -= D.inv_area * D.root_mass;  // every mass enters a walk once
+}
+
+// The part [s0, end) of a walk shared by several warps (s0 a multiple of
+// kCutStep): this ray's terms of the part's nodes.  The decisions at the
+// ancestors of node s0 are taken again (their far-field terms belong to
+// earlier parts), which gives the node where each ray enters the part; false
+// if none does.
+template <bool PHI>
+__device__ __forceinline__ bool walk_strip_part(const TreeDev &D, double rx, double ry, bool valid, StripWarp &W,
+                                                    const ExpTab &tab, int s0, int end, StripAcc &L) {
+  const StripTree T(D);
+  const StripWalk w = strip_begin(rx, ry, valid);
+  int resume = valid ? s0 : 0x7fffffff;
+  const int a = __ldg(D.cutanc + (size_t)kMaxDepth * (s0 / kCutStep) + w.lane);
+  int skip = 0, cls = 2;
+  if (a >= 0) {
+    const double2 *sp = reinterpret_cast<const double2 *>(T.tnodes + a);
+    const double2 c = __ldg(sp);
+    const float4 o = __ldg(reinterpret_cast<const float4 *>(sp + 1));
+    skip = __float_as_int(o.z);
+    cls = strip_class(w, c.x, c.y, o.x, o.y);
+  }
+  unsigned todo = __ballot_sync(kFull, a >= 0 && cls != 2);
+  while (todo) {
+    const int b = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int node = __shfl_sync(kFull, a, b), sk = __shfl_sync(kFull, skip, b), c = __shfl_sync(kFull, cls, b);
+    const GNode *nd = T.nodes + node;
+    const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
+    // every ancestor's subtree holds s0, so the outermost one not opened decides
+    if (c == 1 || !(cx * cx + cy * cy < nd->open2)) resume = max(resume, sk);
+  }
+  const int base = (int)__reduce_min_sync(kFull, valid ? (unsigned)resume : 0x7fffffffu);
+  if (base >= end) return false;
+  strip_run<PHI>(T, w, W, tab, base, end, resume, L);
+  return true;
 }
 
 }  // namespace glb
