@@ -54,17 +54,43 @@ struct DBuf {
   }
 };
 
+// The pool of this device's build scratch.  It keeps up to 256 MB between
+// uses, so that building many trees does not map memory for each (a build
+// takes some twenty buffers); what it holds beyond that goes back to the device
+// at the next synchronisation.
+cudaError_t scratch_pool(cudaMemPool_t *pool);
+
+// Scratch memory from the pool, taken and given back in the order of a stream.
+template <typename T>
+struct ABuf {
+  T *p = nullptr;
+  size_t n = 0;
+  cudaStream_t s;
+  explicit ABuf(cudaStream_t st) : s(st) {}
+  ABuf(const ABuf &) = delete;
+  ABuf &operator=(const ABuf &) = delete;
+  ~ABuf() { release(); }
+  void release() {
+    if (p) cudaFreeAsync(p, s);
+    p = nullptr;
+    n = 0;
+  }
+  cudaError_t alloc(size_t count) {
+    release();
+    if (count == 0) return cudaSuccess;
+    cudaMemPool_t pool;
+    cudaError_t e = scratch_pool(&pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);
+    if (e == cudaSuccess) n = count;
+    return e;
+  }
+};
+
 // TreeQuadParticles built on the device.
 struct Tree {
   TreeDev dev{};
-  DBuf<GNode> nodes;
-  DBuf<GNodeS> snodes;
-  DBuf<TNode> tnodes;
-  DBuf<FNode> fnodes;
-  DBuf<int> cutanc;
-  DBuf<ExpTab> exptab;
-  DBuf<float4> parts;
-  DBuf<float4> prel;
+  DBuf<char> node_mem;      // every array per node, and the exponential's tables
+  DBuf<float4> particles;   // sorted records, then their leaf-relative form
   DBuf<float4> bigs;
   int nnodes = 0;
   size_t nparticles = 0;

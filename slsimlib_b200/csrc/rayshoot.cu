@@ -2404,24 +2404,25 @@ int glb_lens_rayshoot_device_status(glb_lens *l, size_t n, const double *x_dev, 
 }
 
 // Host buffers in and out through the calling thread's staging buffer and
-// stream.  x_on_device: x is already a device array (GridMap positions).
+// stream.  x null: the positions are in the staging buffer's first 2n doubles
+// already (GridMap positions).
 static int rayshoot_host(glb_lens *l, LensWS *w, size_t n, const double *x, const double *zs, double *y,
-                         double *A, int precision, bool x_on_device, const unsigned char *skip = nullptr,
+                         double *A, int precision, const unsigned char *skip = nullptr,
                          unsigned char *status = nullptr) {
   if (n == 0) return 0;
   // staging (doubles): x 2n | zs n | y 2n | A 4n | skip + status (2n bytes, rounded up)
   const size_t flag_words = (skip || status) ? (2 * n + 7) / 8 : 0;
-  size_t need = (x_on_device ? 0 : 2 * n) + (zs ? n : 0) + 6 * n + flag_words;
-  if (w->io.n < need) CKR(w->io.alloc(need));
+  size_t need = 2 * n + (zs ? n : 0) + 6 * n + flag_words;
+  if (x && w->io.n < need) CKR(w->io.alloc(need));
   cudaStream_t s = w->stream;
-  double *dx = x_on_device ? const_cast<double *>(x) : w->io.p;
-  double *dzs = zs ? w->io.p + (x_on_device ? 0 : 2 * n) : nullptr;
-  double *dy = w->io.p + (x_on_device ? 0 : 2 * n) + (zs ? n : 0);
+  double *dx = w->io.p;
+  double *dzs = zs ? w->io.p + 2 * n : nullptr;
+  double *dy = w->io.p + 2 * n + (zs ? n : 0);
   double *dA = dy + 2 * n;
   unsigned char *dflags = reinterpret_cast<unsigned char *>(dA + 4 * n);
   unsigned char *dskip = skip ? dflags : nullptr;
   unsigned char *dstatus = status ? dflags + n : nullptr;
-  if (!x_on_device) CKR(cudaMemcpyAsync(dx, x, 2 * n * sizeof(double), cudaMemcpyHostToDevice, s));
+  if (x) CKR(cudaMemcpyAsync(dx, x, 2 * n * sizeof(double), cudaMemcpyHostToDevice, s));
   if (zs) CKR(cudaMemcpyAsync(dzs, zs, n * sizeof(double), cudaMemcpyHostToDevice, s));
   if (skip) {
     // skipped rays keep the caller's y and A: start from them
@@ -2454,7 +2455,7 @@ int glb_lens_rayshoot_status(glb_lens *l, size_t n, const double *x, const doubl
   if (int rc = set_dev(l->device)) return rc;
   LensWS *w;
   if (int rc = thread_ws(l, &w)) return rc;
-  return rayshoot_host(l, w, n, x, zs, y, A, precision, false, skip, status);
+  return rayshoot_host(l, w, n, x, zs, y, A, precision, skip, status);
 }
 
 int glb_gridmap(glb_lens *l, size_t n1d, const double *center, double range, double *y, double *A, int precision) {
@@ -2466,13 +2467,10 @@ int glb_gridmap(glb_lens *l, size_t n1d, const double *center, double range, dou
   LensWS *w;
   if (int rc = thread_ws(l, &w)) return rc;
   size_t n = n1d * n1d;
-  DBuf<double> dx;
-  CKR(dx.alloc(2 * n));
-  k_grid<<<nblk(n, 256), 256, 0, w->stream>>>(n1d, center[0], center[1], range, dx.p);
+  if (w->io.n < 8 * n) CKR(w->io.alloc(8 * n));
+  k_grid<<<nblk(n, 256), 256, 0, w->stream>>>(n1d, center[0], center[1], range, w->io.p);
   CKR(cudaGetLastError());
-  int rc = rayshoot_host(l, w, n, dx.p, nullptr, y, A, precision, true);
-  CKR(cudaStreamSynchronize(w->stream));
-  return rc;
+  return rayshoot_host(l, w, n, nullptr, nullptr, y, A, precision);
 }
 
 int glb_gridmap_pixelmap(glb_lens *l, size_t n1d, const double *center, double range, int lensvar, double *map,
@@ -2884,8 +2882,8 @@ extern "C" int glb_particles_smoothing(glb_particle *particles, size_t n, int ns
     cudaStream_t s;
     ~StreamGuard() { cudaStreamDestroy(s); }
   } sg{st};
-  DBuf<glb_particle_rec> d_p;
-  DBuf<float> d_size;
+  ABuf<glb_particle_rec> d_p(st);
+  ABuf<float> d_size(st);
   CKR(d_p.alloc(n));
   CKR(d_size.alloc(n));
   if (n) CKR(cudaMemcpyAsync(d_p.p, particles, n * sizeof(glb_particle_rec), cudaMemcpyHostToDevice, st));

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "glb_host.h"
 
@@ -539,6 +540,30 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
+cudaError_t scratch_pool(cudaMemPool_t *pool) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    e = cudaMemPoolCreate(&pools[dev], &props);
+    if (e != cudaSuccess) return e;
+    unsigned long long keep = 256ull << 20;
+    e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) return e;
+  }
+  *pool = pools[dev];
+  return cudaSuccess;
+}
+
 Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, bool want_export,
                   cudaStream_t st, std::unique_ptr<Tree> &out) {
   auto T = std::make_unique<Tree>();
@@ -562,12 +587,12 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   CK(cudaEventCreate(&e1));
   CK(cudaEventRecord(e0, st));
 
-  DBuf<glb_particle_rec> dp;
+  ABuf<glb_particle_rec> dp(st);
   CK(dp.alloc(n));
   CK(cudaMemcpyAsync(dp.p, hp, n * sizeof(glb_particle_rec), cudaMemcpyHostToDevice, st));
 
   // ---- root box (BuildQTreeNB, quadTree.h:297-337)
-  DBuf<unsigned> mm;
+  ABuf<unsigned> mm(st);
   CK(mm.alloc(4));
   unsigned init[4] = {0xffffffffu, 0xffffffffu, 0u, 0u};
   CK(cudaMemcpyAsync(mm.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
@@ -587,8 +612,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   p2[jj] = p1[jj] + lengths[!jj];
 
   // ---- keys + stable sort
-  DBuf<unsigned long long> keys, keys2;
-  DBuf<unsigned> idx, sidx;
+  ABuf<unsigned long long> keys(st), keys2(st);
+  ABuf<unsigned> idx(st), sidx(st);
   CK(keys.alloc(n));
   CK(keys2.alloc(n));
   CK(idx.alloc(n));
@@ -596,7 +621,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   k_keys<<<nblk(n, 256), 256, 0, st>>>(dp.p, n, p1[0], p1[1], p2[0], p2[1], keys.p, idx.p);
   size_t tmp_bytes = 0;
   CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.p, keys2.p, idx.p, sidx.p, (int)n, 0, 64, st));
-  DBuf<char> tmp;
+  ABuf<char> tmp(st);
   CK(tmp.alloc(tmp_bytes));
   CK(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, keys.p, keys2.p, idx.p, sidx.p, (int)n, 0, 64, st));
   keys.release();
@@ -604,8 +629,9 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
 
   // ---- level-by-level expansion
   std::vector<int> off = {0, 1};
-  size_t cap = 1024;
-  DBuf<Slot> slots;
+  // grown below where a tree needs more
+  size_t cap = std::min<size_t>((size_t)1 << 20, std::max<size_t>(1024, 2 * (n / (size_t)prm.bucket)));
+  ABuf<Slot> slots(st);
   CK(slots.alloc(cap));
   Slot root;
   memset(&root, 0, sizeof(root));
@@ -617,7 +643,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   root.pre = 0;
   root.pref = 0;
   CK(cudaMemcpyAsync(slots.p, &root, sizeof(Slot), cudaMemcpyHostToDevice, st));
-  DBuf<int> counters;
+  ABuf<int> counters(st);
   CK(counters.alloc(2));
   for (int L = 0;; ++L) {
     int lo = off[L], hi = off[L + 1];
@@ -633,7 +659,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
     if (need > 0x7fffffffull) return Status::err(-1, "tree too large");
     if (need > cap) {
       size_t ncap = std::max(need, cap * 2);
-      DBuf<Slot> ns;
+      ABuf<Slot> ns(st);
       CK(ns.alloc(ncap));
       CK(cudaMemcpyAsync(ns.p, slots.p, (size_t)hi * sizeof(Slot), cudaMemcpyDeviceToDevice, st));
       std::swap(ns.p, slots.p);
@@ -647,11 +673,12 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   const int nslots = off[nlev];
 
   // ---- moments, bottom-up
-  CK(T->prel.alloc(n));
+  CK(T->particles.alloc(2 * n));
+  float4 *parts = T->particles.p, *prel = parts + n;
   for (int L = nlev - 1; L >= 0; --L) {
     int lo = off[L], hi = off[L + 1];
     k_leaf_moments<<<nblk((long long)(hi - lo) * 32, 256), 256, 0, st>>>(slots.p, lo, hi, dp.p, sidx.p, multimass,
-                                                                          multiradius, prm.theta, T->prel.p);
+                                                                          multiradius, prm.theta, prel);
     k_internal_moments<<<nblk(hi - lo, 256), 256, 0, st>>>(slots.p, lo, hi, prm.theta);
     k_subtree<<<nblk(hi - lo, 256), 256, 0, st>>>(slots.p, lo, hi);
   }
@@ -667,17 +694,16 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   T->nbranches = (size_t)rootb.subf;
 
   // ---- sorted particle records
-  CK(T->parts.alloc(n));
-  k_gather_parts<<<nblk(n, 256), 256, 0, st>>>(dp.p, sidx.p, (int)n, multimass, multiradius, T->parts.p);
+  k_gather_parts<<<nblk(n, 256), 256, 0, st>>>(dp.p, sidx.p, (int)n, multimass, multiradius, parts);
 
   // ---- big-particle lists of internal boxes
-  DBuf<int> pre2slot;
+  ABuf<int> pre2slot(st);
   CK(pre2slot.alloc(nnodes));
   k_pre2slot<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, pre2slot.p);
   int nbig = 0;
   if (multiradius) {
-    DBuf<unsigned> fkey, fval, ckey, cval, skey, sval;
-    DBuf<int> flags, nsel;
+    ABuf<unsigned> fkey(st), fval(st), ckey(st), cval(st), skey(st), sval(st);
+    ABuf<int> flags(st), nsel(st);
     CK(fkey.alloc(n));
     CK(fval.alloc(n));
     CK(flags.alloc(n));
@@ -704,35 +730,40 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
       CK(cub::DeviceRadixSort::SortPairs(tmp.p, tb2, ckey.p, skey.p, cval.p, sval.p, nbig, 0, 32, st));
       k_big_ranges<<<nblk(nbig, 256), 256, 0, st>>>(skey.p, nbig, slots.p, pre2slot.p);
       CK(T->bigs.alloc(nbig));
-      k_gather_bigs<<<nblk(nbig, 256), 256, 0, st>>>(T->parts.p, sval.p, nbig, T->bigs.p);
+      k_gather_bigs<<<nblk(nbig, 256), 256, 0, st>>>(parts, sval.p, nbig, T->bigs.p);
     }
   }
 
   // ---- node array
-  CK(T->nodes.alloc(nnodes));
-  CK(T->snodes.alloc(nnodes));
-  CK(T->tnodes.alloc(nnodes));
-  CK(T->fnodes.alloc(nnodes));
-  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, T->nodes.p, T->snodes.p, T->tnodes.p,
-                                                  T->fnodes.p);
   const int ncut = (nnodes + kCutStep - 1) / kCutStep;
-  CK(T->cutanc.alloc((size_t)ncut * kMaxDepth));
-  CK(T->exptab.alloc(1));
-  k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(T->tnodes.p, ncut, T->cutanc.p);
-  k_exp_tables<<<4, 256, 0, st>>>(T->exptab.p);
-  DBuf<int> dbad;
+  auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t nn = (size_t)nnodes, o_g = 0, o_s = o_g + al(nn * sizeof(GNode)), o_t = o_s + al(nn * sizeof(GNodeS));
+  const size_t o_f = o_t + al(nn * sizeof(TNode)), o_c = o_f + al(nn * sizeof(FNode));
+  const size_t o_e = o_c + al((size_t)ncut * kMaxDepth * sizeof(int));
+  CK(T->node_mem.alloc(o_e + sizeof(ExpTab)));
+  char *nm = T->node_mem.p;
+  GNode *gnodes = (GNode *)(nm + o_g);
+  GNodeS *snodes = (GNodeS *)(nm + o_s);
+  TNode *tnodes = (TNode *)(nm + o_t);
+  FNode *fnodes = (FNode *)(nm + o_f);
+  int *cutanc = (int *)(nm + o_c);
+  ExpTab *exptab = (ExpTab *)(nm + o_e);
+  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes);
+  k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(tnodes, ncut, cutanc);
+  k_exp_tables<<<4, 256, 0, st>>>(exptab);
+  ABuf<int> dbad(st);
   CK(dbad.alloc(1));
   CK(cudaMemsetAsync(dbad.p, 0, sizeof(int), st));
-  if (nnodes > 0) k_check_skips<<<nblk(nnodes, 256), 256, 0, st>>>(T->snodes.p, nnodes, dbad.p);
+  if (nnodes > 0) k_check_skips<<<nblk(nnodes, 256), 256, 0, st>>>(snodes, nnodes, dbad.p);
   int hbad = 0;
   CK(cudaMemcpyAsync(&hbad, dbad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  DBuf<double> phin;
+  ABuf<double> phin(st);
   CK(phin.alloc(8));
   k_phi_node<<<1, 1, 0, st>>>(slots.p, phin.p);
   double hphi[8];
   CK(cudaMemcpyAsync(hphi, phin.p, sizeof(hphi), cudaMemcpyDeviceToHost, st));
   if (want_export) {
-    DBuf<double> ex;
+    ABuf<double> ex(st);
     CK(ex.alloc((size_t)16 * T->nbranches));
     k_export<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, ex.p);
     T->export_rows.resize((size_t)16 * T->nbranches);
@@ -759,15 +790,15 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   T->dev.root_mass = hphi[4];
   T->dev.root_cx = hphi[6];
   T->dev.root_cy = hphi[7];
-  T->dev.nodes = T->nodes.p;
-  T->dev.snodes = T->snodes.p;
-  T->dev.tnodes = T->tnodes.p;
-  T->dev.fnodes = T->fnodes.p;
-  T->dev.cutanc = T->cutanc.p;
-  T->dev.exptab = T->exptab.p;
-  T->dev.parts = T->parts.p;
+  T->dev.nodes = gnodes;
+  T->dev.snodes = snodes;
+  T->dev.tnodes = tnodes;
+  T->dev.fnodes = fnodes;
+  T->dev.cutanc = cutanc;
+  T->dev.exptab = exptab;
+  T->dev.parts = parts;
   T->dev.bigs = T->bigs.p;
-  T->dev.prel = T->prel.p;
+  T->dev.prel = prel;
   T->dev.nnodes = nnodes;
   T->dev.nparticles = (int)n;
   out = std::move(T);
