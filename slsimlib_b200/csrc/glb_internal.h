@@ -67,6 +67,21 @@ struct __align__(16) FNode {
   double mpi, q0pi, q2pi, pad;
 };
 
+// The rows of the split form's group walk (walk_group.cuh): what its
+// classification reads (48 bytes: one round's loads are in flight together, the
+// children among them) and the far-field row (32 bytes: centre as a
+// double-float pair, mass and quadrupole divided by pi).
+struct __align__(16) CNode {
+  double cx, cy, open2;
+  int skip;
+  int info;      // 1: leaf, 2: internal with softened particles, 0: other
+  int child[4];  // preorder indices, -1 beyond the last
+};
+struct __align__(16) FNodeS {
+  float cxh, cyh, cxl, cyl;
+  float mpi, q0pi, q2pi, pad;
+};
+
 // Shared walks (several warps per 32 rays) start at multiples of kCutStep nodes.
 constexpr int kCutStep = 16;
 
@@ -78,6 +93,8 @@ struct ExpTab {
 struct TreeDev {
   const TNode *tnodes;
   const FNode *fnodes;
+  const CNode *cnodes;
+  const FNodeS *fsnodes;
   const int *cutanc;     // kMaxDepth per cut: the ancestors of its node, outermost first, -1 beyond
   const ExpTab *exptab;
   const GNode *nodes;

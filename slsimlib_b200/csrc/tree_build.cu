@@ -386,7 +386,7 @@ __global__ void k_pre2slot(const Slot *s, int nslots, int *pre2slot) {
 }
 
 __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nodes, GNodeS *snodes, TNode *tnodes,
-                             FNode *fnodes) {
+                             FNode *fnodes, CNode *cnodes, FNodeS *fsnodes) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots) return;
   const Slot &b = s[i];
@@ -446,6 +446,19 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   f.start = g.leaf ? g.pstart : g.bstart;
   f.count = g.leaf ? g.pcount : g.bcount;
   snodes[b.pre] = f;
+  fsnodes[b.pre] = FNodeS{f.cxh, f.cyh, f.cxl, f.cyl, f.mpi, f.q0pi, f.q2pi, 0.f};
+  CNode c;
+  c.cx = g.cx;
+  c.cy = g.cy;
+  c.open2 = g.open2;
+  c.skip = g.skip;
+  c.info = g.leaf ? 1 : (g.bcount > 0 ? 2 : 0);
+  int nc = 0;
+  for (int k = 0; k < 4; ++k) c.child[k] = -1;
+  if (b.child >= 0)
+    for (int k = 0; k < 4; ++k)
+      if (s[b.child + k].count > 0) c.child[nc++] = s[b.child + k].pre;
+  cnodes[b.pre] = c;
 }
 
 // The ancestors of every kCutStep-th node, outermost first.
@@ -738,7 +751,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   const int ncut = (nnodes + kCutStep - 1) / kCutStep;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t nn = (size_t)nnodes, o_g = 0, o_s = o_g + al(nn * sizeof(GNode)), o_t = o_s + al(nn * sizeof(GNodeS));
-  const size_t o_f = o_t + al(nn * sizeof(TNode)), o_c = o_f + al(nn * sizeof(FNode));
+  const size_t o_f = o_t + al(nn * sizeof(TNode)), o_n = o_f + al(nn * sizeof(FNode));
+  const size_t o_r = o_n + al(nn * sizeof(CNode)), o_c = o_r + al(nn * sizeof(FNodeS));
   const size_t o_e = o_c + al((size_t)ncut * kMaxDepth * sizeof(int));
   CK(T->node_mem.alloc(o_e + sizeof(ExpTab)));
   char *nm = T->node_mem.p;
@@ -746,9 +760,12 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   GNodeS *snodes = (GNodeS *)(nm + o_s);
   TNode *tnodes = (TNode *)(nm + o_t);
   FNode *fnodes = (FNode *)(nm + o_f);
+  CNode *cnodes = (CNode *)(nm + o_n);
+  FNodeS *fsnodes = (FNodeS *)(nm + o_r);
   int *cutanc = (int *)(nm + o_c);
   ExpTab *exptab = (ExpTab *)(nm + o_e);
-  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes);
+  k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes,
+                                                  cnodes, fsnodes);
   k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(tnodes, ncut, cutanc);
   k_exp_tables<<<4, 256, 0, st>>>(exptab);
   ABuf<int> dbad(st);
@@ -794,6 +811,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   T->dev.snodes = snodes;
   T->dev.tnodes = tnodes;
   T->dev.fnodes = fnodes;
+  T->dev.cnodes = cnodes;
+  T->dev.fsnodes = fsnodes;
   T->dev.cutanc = cutanc;
   T->dev.exptab = exptab;
   T->dev.parts = parts;

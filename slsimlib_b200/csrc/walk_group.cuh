@@ -37,25 +37,25 @@ struct GroupLists {
   int leaf[kGL];
   int big[kGB];
   int mixed[kGM];
-  float4 rows[4][96];  // per warp: the three rows of 32 far cells
+  float4 rows[4][64];  // per warp: the rows of 32 far cells, or a leaf's particles
   int qhead, qtail, nfar, nleaf, nbig, nmixed, done, any;
   double box[4];  // xmin, xmax, ymin, ymax of the block's valid rays
 };
 
 // A far-field term into the FP32 partial sums (far_term without the flush
-// check: the caller flushes every 32 terms).  Invalid lanes add garbage that
-// their caller never reads back (their totals are dropped).
-__device__ __forceinline__ void far_sum(const float4 &c1, const float4 &c2, float2 d, bool screen, float ns2l,
-                                        float piaf, F32Acc &fa) {
+// check: the caller flushes every 32 terms).  m: {mass/pi, q0/pi, q2/pi};
+// q1 = -q0.  Invalid lanes add garbage that their caller never reads back
+// (their totals are dropped).
+__device__ __forceinline__ void far_sum(const float4 &m, float2 d, bool screen, float ns2l, float piaf, F32Acc &fa) {
   const float2 dd = __fmul2_rn(d, d);
   const float r2f = dd.x + dd.y;
   const float scr = screen ? ex2_approx(r2f * ns2l) : 1.0f;
   const float ir2 = rcp_approx(r2f);
-  const float ms = c1.z * scr;
+  const float ms = m.x * scr;
   const float sir4 = scr * ir2 * ir2;
-  const float qx = fmaf(c2.w, d.x, c2.y * d.y), qy = fmaf(c2.x, d.y, c2.y * d.x);
+  const float qx = fmaf(m.y, d.x, m.z * d.y), qy = fmaf(-m.y, d.y, m.z * d.x);
   const float qd = fmaf(qx, d.x, qy * d.y);
-  const float t = fmaf(c1.z, piaf, -ms * ir2) + 4.f * qd * sir4 * ir2;
+  const float t = fmaf(m.x, piaf, -ms * ir2) + 4.f * qd * sir4 * ir2;
   fa.a = __ffma2_rn(f2(t), d, fa.a);
   fa.a = __ffma2_rn(f2(-sir4), make_float2(qx, qy), fa.a);
   fa.g = __ffma2_rn(f2(-ms * ir2 * ir2), make_float2(dd.x - dd.y, d.x * d.y), fa.g);
@@ -78,23 +78,25 @@ __device__ __forceinline__ bool group_classify(const TreeDev &T, GroupLists &G) 
     }
     if (nfar + 32 > kGF || nleaf + 32 > kGL || nbig + 32 > kGB || nmixed + 32 > kGM) break;
     const int cnt = min(32, tail - head);
-    int node = -1, cat = 0, skipn = 0, bc = 0, nch = 0;  // cat: 1 accept, 2 open leaf, 3 open internal, 4 mixed
+    int node = -1, cat = 0, bc = 0, nch = 0;  // cat: 1 accept, 2 open leaf, 3 open internal, 4 mixed
+    int4 ch = make_int4(-1, -1, -1, -1);
     if (lane < cnt) {
       node = G.q[(head + lane) & (kGQ - 1)];
-      const GNode &nd = T.nodes[node];
-      const double cx = nd.cx, cy = nd.cy, o2 = nd.open2;
+      const double2 *row = reinterpret_cast<const double2 *>(T.cnodes + node);
+      const double2 c = __ldg(row), o = __ldg(row + 1);
+      ch = __ldg(reinterpret_cast<const int4 *>(row + 2));
+      const double cx = c.x, cy = c.y, o2 = o.x;
+      const int info = __double2hiint(o.y);
       const double nx = cx < xmin ? xmin - cx : (cx > xmax ? cx - xmax : 0.0);
       const double ny = cy < ymin ? ymin - cy : (cy > ymax ? cy - ymax : 0.0);
       const double fx = fmax(fabs(cx - xmin), fabs(cx - xmax)), fy = fmax(fabs(cy - ymin), fabs(cy - ymax));
       const double dmin2 = nx * nx + ny * ny, dmax2 = fx * fx + fy * fy;
-      skipn = nd.skip;
       if (dmin2 >= o2 * (1.0 + 1e-12)) {
         cat = 1;
       } else if (dmax2 < o2 * (1.0 - 1e-12)) {
-        cat = nd.leaf ? 2 : 3;
-        bc = nd.leaf ? 0 : nd.bcount;
-        if (cat == 3)
-          for (int c = node + 1; c < skipn; c = T.nodes[c].skip) ++nch;
+        cat = info == 1 ? 2 : 3;
+        bc = info == 2 ? 1 : 0;
+        nch = (ch.x >= 0) + (ch.y >= 0) + (ch.z >= 0) + (ch.w >= 0);  // a leaf has none
       } else {
         cat = 4;
       }
@@ -111,8 +113,11 @@ __device__ __forceinline__ bool group_classify(const TreeDev &T, GroupLists &G) 
     if ((tail - head) + total > kGQ) {
       if (cat == 3) cat = 4;
     } else if (cat == 3) {
-      int pos = tail + incl - nch;
-      for (int c = node + 1; c < skipn; c = T.nodes[c].skip) G.q[(pos++) & (kGQ - 1)] = c;
+      const int pos = tail + incl - nch;
+      if (ch.x >= 0) G.q[pos & (kGQ - 1)] = ch.x;
+      if (ch.y >= 0) G.q[(pos + 1) & (kGQ - 1)] = ch.y;
+      if (ch.z >= 0) G.q[(pos + 2) & (kGQ - 1)] = ch.z;
+      if (ch.w >= 0) G.q[(pos + 3) & (kGQ - 1)] = ch.w;
     }
     if ((tail - head) + total <= kGQ) tail += total;
     unsigned m = __ballot_sync(kFull, cat == 1);
@@ -247,19 +252,18 @@ __device__ __forceinline__ void walk_group(const TreeDev &T, const double *rxy, 
       for (int i0 = 0; i0 < nfar; i0 += 32) {
         const int cnt = min(32, nfar - i0);
         if (lane < cnt) {
-          const float4 *sp = reinterpret_cast<const float4 *>(T.snodes + G.far[i0 + lane]);
-          wrow[3 * lane] = __ldg(sp);
-          wrow[3 * lane + 1] = __ldg(sp + 1);
-          wrow[3 * lane + 2] = __ldg(sp + 2);
+          const float4 *sp = reinterpret_cast<const float4 *>(T.fsnodes + G.far[i0 + lane]);
+          wrow[2 * lane] = __ldg(sp);
+          wrow[2 * lane + 1] = __ldg(sp + 1);
         }
         __syncwarp();
         if (valid && fa.cnt > 0) fa.flush(acc);
-#pragma unroll 8  // 638 ms per light-cone step; 4: 644, 2: 651
+#pragma unroll 8  // ms per light-cone step: 492; 4: 498, 16: 498
         for (int j = 0; j < cnt; ++j) {
-          const float4 c0 = wrow[3 * j], c1 = wrow[3 * j + 1], c2 = wrow[3 * j + 2];
+          const float4 c0 = wrow[2 * j], m = wrow[2 * j + 1];
           const float2 d =
               __fadd2_rn(__fadd2_rn(make_float2(c0.x, c0.y), nrh), __fadd2_rn(make_float2(c0.z, c0.w), nrl));
-          far_sum(c1, c2, d, screen, ns2l, piaf, fa);
+          far_sum(m, d, screen, ns2l, piaf, fa);
         }
         if (valid) fa.flush(acc);
         __syncwarp();
