@@ -50,6 +50,8 @@ struct __align__(16) GNodeS {
   float cxh, cyh, cxl, cyl;
   float open2, near2, mpi, open_band;
   float q1pi, q2pi, width_ru, q0pi;
+  // leaf: the bits of a squared distance of the centre (never 0) beyond which
+  // none of its particles is within its near-field radius, 0 for an internal node
   int skip, leaf, start, count;  // leaf: particle range; internal: big-particle range
 };
 

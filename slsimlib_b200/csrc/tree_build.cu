@@ -40,7 +40,9 @@ struct Slot {
   double r2crit;
   int start, count, child, level;
   int sub, pre, subf, pref;
-  int nbig, bstart, pad0, pad1;
+  int nbig, bstart;
+  float clear2;  // leaf: beyond this squared distance of the centre every particle is a point mass
+  int pad;
 };
 
 #define CK(call)                                                                     \
@@ -245,13 +247,18 @@ __global__ void k_leaf_moments(Slot *s, int lo, int hi, const glb_particle_rec *
   // mass, -mass/pi and the squared near-field radius (two softening lengths,
   // widened by 2.5e-5 against FP32 rounding; at least 1e-12 so that
   // coincident particles are sent to FP64)
+  double far = 0;
   for (int k = b.start + lane; k < b.start + b.count; k += 32) {
     unsigned id = sidx[k];
     const double sz = (double)p[multiradius ? id : 0].Size;
     prel[k] = make_float4((float)((double)p[id].x[0] - cx), (float)((double)p[id].x[1] - cy),
                           (float)(-(double)p[multimass ? id : 0].Mass / kPi), (float)fmax(4.0001 * sz * sz, 1e-12));
+    const double dx = (double)p[id].x[0] - cx, dy = (double)p[id].x[1] - cy;
+    far = fmax(far, sqrt(dx * dx + dy * dy) + sqrt(fmax(4.0001 * sz * sz, 1e-12)));
   }
+  for (int o = 16; o > 0; o >>= 1) far = fmax(far, __shfl_xor_sync(kFullMask, far, o));
   if (lane == 0) {
+    b.clear2 = __double2float_ru(far * far * (1.0 + 2e-5));  // (FP32 rounding of the rays' offsets: 2e-7)
     b.mass = M;
     b.absm = A;
     b.comx = cx;
@@ -442,7 +449,7 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   f.width_ru = __double2float_ru(g.width);
   f.open_band = kAmbiguous * f.open2;
   f.skip = g.skip;
-  f.leaf = g.leaf;
+  f.leaf = g.leaf ? __float_as_int(b.clear2) : 0;
   f.start = g.leaf ? g.pstart : g.bstart;
   f.count = g.leaf ? g.pcount : g.bcount;
   snodes[b.pre] = f;

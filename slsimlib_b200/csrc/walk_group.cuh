@@ -185,11 +185,17 @@ __device__ __forceinline__ void group_subtree(const TreeDev &T, const double *rx
       const int p0 = c3.z, p1 = p0 + c3.w;
       const float wu = __ldg(sp + 2).z;
       if (open && (nearc ? fa.cnt > 0 : fa.cnt + min(c3.w, 32) > 32)) fa.flush(acc);
+      const bool clear = !__any_sync(kFull, open && r2f < __int_as_float(c3.y));
       for (int q0 = p0; q0 < p1; q0 += 32) {
         const int q1 = min(q0 + 32, p1);
         // the whole warp is here (some lane opened the leaf): stage its particles
         if (q0 + lane < q1) wrow[lane] = __ldg(T.prel + q0 + lane);
         __syncwarp();
+        if (clear) {
+          if (open)
+#pragma unroll 4
+            for (int p = 0; p < q1 - q0; ++p) clear_term(wrow[p], d, screen, ns2l, piaf, sheet, fa);
+        } else
         for (int p = q0; p < q1; ++p) {
           const float4 P = wrow[p - q0];
           if (open) leaf_term(T, P, p, d, rxy, nearc, screen, s2f, ns2l, piaf, sheet, wu, node, fa, acc);
@@ -285,12 +291,17 @@ __device__ __forceinline__ void walk_group(const TreeDev &T, const double *rxy, 
           if (fabsf(e) <= kAmbiguous * c1.y) nearc = node_test_f64(T.nodes + node, rx, ry, 1);
         }
         const int p0 = c3.z, p1 = p0 + c3.w;
+        const bool clear = !__any_sync(kFull, valid && r2f < __int_as_float(c3.y));
         if (valid && (nearc ? fa.cnt > 0 : fa.cnt + min(c3.w, 32) > 32)) fa.flush(acc);
         for (int q0 = p0; q0 < p1; q0 += 32) {
           const int q1 = min(q0 + 32, p1);
           // the chunk's particles, one per lane, into the warp's rows
           if (q0 + lane < q1) wrow[lane] = __ldg(T.prel + q0 + lane);
           __syncwarp();
+          if (clear) {  // (lanes without a ray add garbage nobody reads)
+#pragma unroll 4
+            for (int p = 0; p < q1 - q0; ++p) clear_term(wrow[p], d, screen, ns2l, piaf, sheet, fa);
+          } else
           for (int p = q0; p < q1; ++p) {
             const float4 P = wrow[p - q0];
             if (valid) leaf_term(T, P, p, d, rxy, nearc, screen, s2f, ns2l, piaf, sheet, wu, node, fa, acc);

@@ -152,6 +152,25 @@ __device__ __forceinline__ void softened_f32(float2 x, float r2, float m, float 
   fa.k = fmaf(m, sg, fa.k);
 }
 
+// A leaf particle as a point mass: x its offset, r2 = |x|^2.
+__device__ __forceinline__ void point_term(float4 P, float2 x, float2 xx, float r2, bool screen, float ns2l,
+                                           float piaf, bool sheet, F32Acc &fa) {
+  const float scr = screen ? ex2_approx(r2 * ns2l) : 1.0f;
+  const float ir2 = rcp_approx(r2);
+  const float npre = P.z * scr * ir2;  // -mass scr / (pi r^2)
+  fa.a = __ffma2_rn(f2(npre), x, fa.a);
+  fa.g = __ffma2_rn(f2(npre * ir2), make_float2(xx.x - xx.y, x.x * x.y), fa.g);
+  if (sheet) fa.a = __ffma2_rn(f2(-piaf * P.z), x, fa.a);  // inv_area * mass * x
+}
+// The same for a particle of a leaf that is clear of the ray (GNodeS::leaf):
+// no near-field test, so that the loop over the leaf has no branch.
+__device__ __forceinline__ void clear_term(float4 P, float2 d, bool screen, float ns2l, float piaf, bool sheet,
+                                           F32Acc &fa) {
+  const float2 x = __fadd2_rn(make_float2(P.x, P.y), d);
+  const float2 xx = __fmul2_rn(x, x);
+  point_term(P, x, xx, xx.x + xx.y, screen, ns2l, piaf, sheet, fa);
+}
+
 // b_spline_profile (include/quadTree.h:147-190) in FP32, for the plain FP32
 // form only.
 __device__ __forceinline__ void bspline_f32(float x0, float x1, float r, float Mass, float size, float *f) {
@@ -274,8 +293,18 @@ __device__ __forceinline__ void walk_split(const TreeDev &T, double rx, double r
       // p99.9 of a softened, sheeted tree from under 1e-5 to 1.4e-5).
       // Leaves of more than 32 particles go in chunks of 32.
       if (!PURE && open && ((nearc || !MERGE) ? fa.cnt > 0 : fa.cnt + min(c3.w, 32) > 32)) fa.flush(acc);
+      const bool clear = !PURE && !__any_sync(kFull, open && r2f < __int_as_float(c3.y));
       for (int q0 = p0; q0 < p1; q0 += 32) {
         const int q1 = min(q0 + 32, p1);
+        if (clear) {
+          if (open) {
+#pragma unroll 4
+            for (int p = q0; p < q1; ++p) clear_term(__ldg(T.prel + p), d, screen, ns2l, piaf, sheet, fa);
+            fa.cnt += q1 - q0;
+            if (nearc || !MERGE || q1 < p1) fa.flush(acc);
+          }
+          continue;
+        }
 #pragma unroll 2  // two independent particles in flight (measured: 6.6 % faster at 64 registers)
         for (int p = q0; p < q1; ++p) {
           const float4 P = __ldg(T.prel + p);  // {x - cx, y - cy, -mass/pi, near radius^2}
@@ -419,12 +448,7 @@ __device__ __forceinline__ void leaf_term(const TreeDev &T, float4 P, int p, flo
       return;
     }
   }
-  const float scr = screen ? ex2_approx(r2 * ns2l) : 1.0f;
-  const float ir2 = rcp_approx(r2);
-  const float npre = P.z * scr * ir2;
-  fa.a = __ffma2_rn(f2(npre), x, fa.a);
-  fa.g = __ffma2_rn(f2(npre * ir2), make_float2(xx.x - xx.y, x.x * x.y), fa.g);
-  if (sheet) fa.a = __ffma2_rn(f2(-piaf * P.z), x, fa.a);
+  point_term(P, x, xx, r2, screen, ns2l, piaf, sheet, fa);
 }
 
 // The split walk for two rays per lane (a warp walks 64 neighbouring rays):
@@ -515,8 +539,27 @@ __device__ __forceinline__ void walk_split2(const TreeDev &T, const double *rxy,
       const float wu = __ldg(sp + 2).z;
       if (open0 && fa0.cnt) fa0.flush(acc0);
       if (open1 && fa1.cnt) fa1.flush(acc1);
+      const float clear2 = __int_as_float(c3.y);
+      const bool clear = !__any_sync(kFull, (open0 && r2f0 < clear2) || (open1 && r2f1 < clear2));
       for (int q0 = p0; q0 < p1; q0 += 32) {
         const int q1 = min(q0 + 32, p1);
+        if (clear) {
+          if (open0 && open1) {
+#pragma unroll 2
+            for (int p = q0; p < q1; ++p) {
+              const float4 P = __ldg(T.prel + p);
+              clear_term(P, d0, screen, ns2l, piaf, sheet, fa0);
+              clear_term(P, d1, screen, ns2l, piaf, sheet, fa1);
+            }
+          } else if (open0) {
+            for (int p = q0; p < q1; ++p) clear_term(__ldg(T.prel + p), d0, screen, ns2l, piaf, sheet, fa0);
+          } else if (open1) {
+            for (int p = q0; p < q1; ++p) clear_term(__ldg(T.prel + p), d1, screen, ns2l, piaf, sheet, fa1);
+          }
+          if (open0) fa0.flush(acc0);
+          if (open1) fa1.flush(acc1);
+          continue;
+        }
         for (int p = q0; p < q1; ++p) {
           const float4 P = __ldg(T.prel + p);
           if (open0) leaf_term(T, P, p, d0, rxy, nearc0, screen, s2f, ns2l, piaf, sheet, wu, node, fa0, acc0);
