@@ -447,8 +447,10 @@ __device__ __forceinline__ void particle_halo_f64(const TreeDev &T, double rx, d
                                                   const ExpTab &tab, double *acc, int A) {
   const int im = T.periodic ? 1 : 0;
   for (int i = -im; i <= im; ++i)
-    for (int j = -im; j <= im; ++j)
-      walk_strip<PHI>(T, im ? rx + i * T.period_x : rx, im ? ry + j * T.period_y : ry, valid, W, tab, acc, A);
+    for (int j = -im; j <= im; ++j) {
+      const double x = im ? rx + i * T.period_x : rx, y = im ? ry + j * T.period_y : ry;
+      walk_strip<PHI, 1>(T, &x, &y, &valid, W, tab, acc, A);
+    }
 }
 
 // Analytic halo of a plane at one position; kept out of line so that the rare
@@ -717,6 +719,63 @@ __global__ void __launch_bounds__(128, 5) k_plane_step_f64(const __grid_constant
   }
   if (valid) recursion_step(a, k, al0, al1, kap, g0, g1);
 }
+// The same for a plane with one particle halo, two rays per lane (pair_walks):
+// a warp walks 64 neighbouring rays, so that strips, staged rows and leaves
+// serve twice as many, and each lane has two independent chains of FP64
+// instructions in flight.  Every ray's result is k_plane_step_f64's.  512^2
+// rays on 2^18 particles: 7.98 -> 7.09 ms; FP64 pipe 57 %, issue 57 % at 14
+// warps per SM (128 registers; 96 registers 8.4 ms).
+__global__ void __launch_bounds__(128, 4) k_plane_step_f64_pair(const __grid_constant__ StepArgs a) {
+  __shared__ StripBlock<128> S;
+  __shared__ double sacc[12 * 128];
+  const int t = threadIdx.x;
+  strip_exp_table(S.tab, a.exptab);
+  __syncthreads();
+  const size_t k0 = blockIdx.x * (size_t)256 + (t >> 5) * 64 + (t & 31);
+  double rx[2], ry[2];
+  bool valid[2];
+  const double D = a.planes[a.j].Dphys;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const size_t k = k0 + 32 * r;
+    const bool inrange = k < a.n;
+    valid[r] = inrange && a.j < ((a.jmax_ray && inrange) ? a.jmax_ray[k] : a.jmax);
+    rx[r] = valid[r] ? __dmul_rn(a.st[k], D) - a.tree_px : 0.0;
+    ry[r] = valid[r] ? __dmul_rn(a.st[a.n + k], D) - a.tree_py : 0.0;
+  }
+  if (!__any_sync(kFull, valid[0] || valid[1])) return;
+  double *acc = sacc + t;
+  for (int c = 0; c < 12; ++c) acc[c * 128] = 0.0;
+  walk_strip<false, 2>(a.tree, rx, ry, valid, S.warp[t >> 5], S.tab, acc, 128);
+  const PlaneDev &P = a.planes[a.j];
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
+    const size_t k = k0 + 32 * r;
+    if (!(k < a.n && a.j < (a.jmax_ray ? a.jmax_ray[k] : a.jmax))) continue;
+    const double xx0 = __dmul_rn(a.st[k], P.Dphys), xx1 = __dmul_rn(a.st[a.n + k], P.Dphys);
+    double al0 = 0, al1 = 0, kap = 0, g0 = 0, g1 = 0;
+    for (int h = 0; h < P.nhalo; ++h) {
+      const HaloDev *H = a.halos + P.halo0 + h;
+      if (H->kind == HALO_PARTICLES) {
+        const double *o = acc + 6 * r * 128;
+        al0 += o[0];
+        al1 += o[128];
+        kap += o[256];
+        g0 += o[384];
+        g1 += o[512];
+      } else {
+        const Force5 f = analytic_halo(H, &a.tab, xx0 - H->px, xx1 - H->py);
+        al0 -= f.a0;
+        al1 -= f.a1;
+        kap += f.k;
+        g0 += f.g0;
+        g1 += f.g1;
+      }
+    }
+    recursion_step(a, k, al0, al1, kap, g0, g1);
+  }
+}
+
 // Shared walks: calls of too few rays to fill the GPU with one warp per 32 rays
 // split every walk over warps that each take a range of the tree's nodes
 // (walk_strip_part); a second kernel adds the parts of a ray in node order.
@@ -1386,6 +1445,22 @@ constexpr size_t kPlanePartsMax = (size_t)1 << 16;
 // weighs more than in a lens's planes).
 constexpr size_t kForcePartsMax = (size_t)1 << 18;
 
+// Whether a plane step of n rays walks two rays per lane.  A wave of the
+// one-ray kernel (5 blocks of 128 rays an SM) takes about 5.4 time units where
+// one of the two-ray kernel (4 blocks of 256) takes 7.6, and calls of a few
+// waves pay for whole ones.  Two planes of 2^17.6 particles in all, one / two
+// rays, ms: 66,049 rays 7.96 / 9.41, 131,044 11.6 / 9.95, 184,900 13.3 / 13.9,
+// 262,144 14.8 / 12.8, 524,176 29.9 / 26.3.
+bool pair_walks(size_t n) {
+  static const int sms = [] {
+    int dev = 0, v = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  const size_t one = (size_t)sms * 5 * 128, two = (size_t)sms * 4 * 256;
+  return 7.6 * (double)((n + two - 1) / two) < 5.4 * (double)((n + one - 1) / one);
+}
+
 // The particle halo of a plane that holds exactly one and no field plane
 // (periodic trees, which LensHaloParticles never builds, are left to the
 // general kernels), or null.
@@ -1500,6 +1575,8 @@ int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int prec
       k_plane_step<false, true><<<nb, 128, 0, s>>>(a);
     else if (l->has_nfw)
       k_plane_step<false, false><<<nb, 128, 0, s>>>(a);
+    else if (ptree && pair_walks(n))
+      k_plane_step_f64_pair<<<nblk(n, 256), 128, 0, s>>>(a);
     else if (ptree)
       k_plane_step_f64<true><<<nb, 128, 0, s>>>(a);
     else

@@ -126,13 +126,33 @@ __device__ __forceinline__ void strip_soften(const TreeDev *T, double x0, double
   if (PHI) L.p += o.v[5];
 }
 
-// The warp's constants of one walk.
+// The warp's constants of one walk.  R: rays per lane.
+template <int R>
 struct StripWalk {
-  double rx, ry;   // this lane's ray
-  double bx, by;   // centre of the box of the warp's valid rays
-  float hx, hy;    // its half extents, rounded up
-  unsigned vmask;  // lanes with a valid ray
+  double rx[R], ry[R];  // this lane's rays
+  double bx, by;        // centre of the box of the warp's valid rays
+  float hx, hy;         // its half extents, rounded up
+  unsigned vmask[R];    // lanes whose r-th ray is valid
   int lane;
+  __device__ __forceinline__ bool has(const unsigned *m, int r) const { return m[r] >> lane & 1u; }
+};
+
+// One mask of lanes per ray of a lane.
+template <int R>
+struct StripMask {
+  unsigned m[R];
+  __device__ __forceinline__ bool any() const {
+    unsigned a = m[0];
+#pragma unroll
+    for (int r = 1; r < R; ++r) a |= m[r];
+    return a != 0u;
+  }
+  __device__ __forceinline__ bool is(const unsigned *v) const {
+    bool e = true;
+#pragma unroll
+    for (int r = 0; r < R; ++r) e = e && m[r] == v[r];
+    return e;
+  }
 };
 
 // FP32 keys in the order of their values, for the integer warp reductions.
@@ -145,18 +165,26 @@ __device__ __forceinline__ float key_f(int k) { return __int_as_float(k ^ ((k >>
 // The box is that of the rays rounded outwards to FP32 (a warp's rays spread
 // far wider than that); rays that are not finite stay out of it (whatever their
 // nodes' classes, their sums are not finite).
-__device__ __forceinline__ StripWalk strip_begin(double rx, double ry, bool valid) {
-  StripWalk w;
-  w.rx = rx;
-  w.ry = ry;
+template <int R>
+__device__ __forceinline__ StripWalk<R> strip_begin(const double *rx, const double *ry, const bool *valid) {
+  StripWalk<R> w;
   w.lane = threadIdx.x & 31;
-  w.vmask = __ballot_sync(kFull, valid);
-  const bool in = valid && isfinite(rx) && isfinite(ry);
   constexpr float kBig = 1e30f;
-  const float x0 = key_f(__reduce_min_sync(kFull, f_key(in ? __double2float_rd(rx) : kBig)));
-  const float x1 = key_f(__reduce_max_sync(kFull, f_key(in ? __double2float_ru(rx) : -kBig)));
-  const float y0 = key_f(__reduce_min_sync(kFull, f_key(in ? __double2float_rd(ry) : kBig)));
-  const float y1 = key_f(__reduce_max_sync(kFull, f_key(in ? __double2float_ru(ry) : -kBig)));
+  float a = kBig, b = -kBig, c = kBig, d = -kBig;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    w.rx[r] = rx[r];
+    w.ry[r] = ry[r];
+    w.vmask[r] = __ballot_sync(kFull, valid[r]);
+    if (valid[r] && isfinite(rx[r]) && isfinite(ry[r])) {
+      a = fminf(a, __double2float_rd(rx[r]));
+      b = fmaxf(b, __double2float_ru(rx[r]));
+      c = fminf(c, __double2float_rd(ry[r]));
+      d = fmaxf(d, __double2float_ru(ry[r]));
+    }
+  }
+  const float x0 = key_f(__reduce_min_sync(kFull, f_key(a))), x1 = key_f(__reduce_max_sync(kFull, f_key(b)));
+  const float y0 = key_f(__reduce_min_sync(kFull, f_key(c))), y1 = key_f(__reduce_max_sync(kFull, f_key(d)));
   w.bx = 0.5 * ((double)x0 + (double)x1);
   w.by = 0.5 * ((double)y0 + (double)y1);
   w.hx = __double2float_ru(0.5 * ((double)x1 - (double)x0)) * 1.000001f;
@@ -167,7 +195,8 @@ __device__ __forceinline__ StripWalk strip_begin(double rx, double ry, bool vali
 // 1: accepted by all, 2: opened by all, 0: mixed.  olo, ohi: the squared
 // opening radius less and plus the margin.  The half extents are rounded up
 // by 1e-6, which covers the rounding of dx - hx where the two are close.
-__device__ __forceinline__ int strip_class(const StripWalk &w, double cx, double cy, float olo, float ohi) {
+template <int R>
+__device__ __forceinline__ int strip_class(const StripWalk<R> &w, double cx, double cy, float olo, float ohi) {
   const float dx = fabsf((float)(cx - w.bx)), dy = fabsf((float)(cy - w.by));
   const float nx = fmaxf(dx - w.hx, 0.f), ny = fmaxf(dy - w.hy, 0.f), fx = dx + w.hx, fy = dy + w.hy;
   return nx * nx + ny * ny >= ohi ? 1 : (fx * fx + fy * fy < olo ? 2 : 0);
@@ -175,33 +204,37 @@ __device__ __forceinline__ int strip_class(const StripWalk &w, double cx, double
 
 // The cnt queued far-field rows for every valid lane, or with MASKED for the
 // lanes of each row's mask.
-template <bool PHI, bool SCREEN, bool SHEET, bool MASKED>
-__device__ __forceinline__ void strip_far_rows(const StripTree &T, const StripWalk &w, const StripWarp &W, int cnt,
-                                               const ExpTab &tab, StripAcc &L) {
+template <bool PHI, bool SCREEN, bool SHEET, bool MASKED, int R>
+__device__ __forceinline__ void strip_far_rows(const StripTree &T, const StripWalk<R> &w, const StripWarp &W, int cnt,
+                                               const ExpTab &tab, StripAcc *LL) {
   const double s2 = T.s2, pia = T.pia;
   const double2 *row = W.far;
 #pragma unroll 1
   for (int j = 0; j < cnt; ++j, row += 3) {
     const double2 c = row[0], mq = row[1], qm = row[2];
-    const double dx = c.x - w.rx, dy = c.y - w.ry;
-    const double xx = __dmul_rn(dx, dx), r2 = __fma_rn(dy, dy, xx);
-    const double ir2 = strip_rcp(r2);
-    const double si = SCREEN ? __dmul_rn(strip_exp_neg(__dmul_rn(r2, s2), tab), ir2) : ir2;
-    const double a = __dmul_rn(mq.x, si), s4 = __dmul_rn(si, ir2);  // mass/pi scr/r^2, scr/r^4
-    const double qx = __fma_rn(mq.y, dx, __dmul_rn(qm.x, dy)), qy = __fma_rn(qm.x, dx, -__dmul_rn(mq.y, dy));
-    const double e = __dmul_rn(__dmul_rn(4.0, s4), __dmul_rn(__fma_rn(qx, dx, __dmul_rn(qy, dy)), ir2));
-    const double t = SHEET ? __fma_rn(mq.x, pia, -a) : -a;
-    const double gc = __dmul_rn(a, ir2), dd = __fma_rn(-dy, dy, xx), xy = __dmul_rn(dx, dy);
-    if (!MASKED || ((unsigned)__double2loint(qm.y) >> w.lane & 1u)) {
-      L.a0 = __fma_rn(e, dx, __fma_rn(-s4, qx, __fma_rn(t, dx, L.a0)));
-      L.a1 = __fma_rn(e, dy, __fma_rn(-s4, qy, __fma_rn(t, dy, L.a1)));
-      L.g0 = __fma_rn(-gc, dd, L.g0);
-      L.g1 = __fma_rn(-gc, xy, L.g1);
-      if (PHI) {
-        const double scr = __dmul_rn(si, r2) * (1.0 / kPi);
-        L.p += 0.5 * T.dev->phi_mass * log(r2) * scr -
-               0.5 * (T.dev->phi_q0 * xx + T.dev->phi_q1 * dy * dy + 2 * T.dev->phi_q2 * xy) * (1.0 / kPi) * s4 -
-               0.5 * pia * mq.x * r2;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      StripAcc &L = LL[r];
+      const double dx = c.x - w.rx[r], dy = c.y - w.ry[r];
+      const double xx = __dmul_rn(dx, dx), r2 = __fma_rn(dy, dy, xx);
+      const double ir2 = strip_rcp(r2);
+      const double si = SCREEN ? __dmul_rn(strip_exp_neg(__dmul_rn(r2, s2), tab), ir2) : ir2;
+      const double a = __dmul_rn(mq.x, si), s4 = __dmul_rn(si, ir2);  // mass/pi scr/r^2, scr/r^4
+      const double qx = __fma_rn(mq.y, dx, __dmul_rn(qm.x, dy)), qy = __fma_rn(qm.x, dx, -__dmul_rn(mq.y, dy));
+      const double e = __dmul_rn(__dmul_rn(4.0, s4), __dmul_rn(__fma_rn(qx, dx, __dmul_rn(qy, dy)), ir2));
+      const double t = SHEET ? __fma_rn(mq.x, pia, -a) : -a;
+      const double gc = __dmul_rn(a, ir2), dd = __fma_rn(-dy, dy, xx), xy = __dmul_rn(dx, dy);
+      if (!MASKED || ((unsigned)(r == 0 ? __double2loint(qm.y) : __double2hiint(qm.y)) >> w.lane & 1u)) {
+        L.a0 = __fma_rn(e, dx, __fma_rn(-s4, qx, __fma_rn(t, dx, L.a0)));
+        L.a1 = __fma_rn(e, dy, __fma_rn(-s4, qy, __fma_rn(t, dy, L.a1)));
+        L.g0 = __fma_rn(-gc, dd, L.g0);
+        L.g1 = __fma_rn(-gc, xy, L.g1);
+        if (PHI) {
+          const double scr = __dmul_rn(si, r2) * (1.0 / kPi);
+          L.p += 0.5 * T.dev->phi_mass * log(r2) * scr -
+                 0.5 * (T.dev->phi_q0 * xx + T.dev->phi_q1 * dy * dy + 2 * T.dev->phi_q2 * xy) * (1.0 / kPi) * s4 -
+                 0.5 * pia * mq.x * r2;
+        }
       }
     }
   }
@@ -214,36 +247,40 @@ struct StripQueue {
   bool masked = false;
 };
 
-// Queues the far-field rows of the strip positions in `who` (r0, r1, r2: this
+// Queues the far-field rows of the strip positions in `who` (r0, r1, q2: this
 // lane's row; fm: the lanes that take it).
-__device__ __forceinline__ void strip_push(const StripWalk &w, StripWarp &W, StripQueue &q, unsigned who, double2 r0,
-                                           double2 r1, double q2, unsigned fm) {
+template <int R>
+__device__ __forceinline__ void strip_push(const StripWalk<R> &w, StripWarp &W, StripQueue &q, unsigned who, double2 r0,
+                                           double2 r1, double q2, const StripMask<R> &fm) {
   if (who >> w.lane & 1u) {
     double2 *row = W.far + 3 * (q.n + __popc(who & ((1u << w.lane) - 1u)));
     row[0] = r0;
     row[1] = r1;
-    row[2] = make_double2(q2, __hiloint2double(0, (int)fm));
+    row[2] = make_double2(q2, __hiloint2double(R > 1 ? (int)fm.m[R - 1] : 0, (int)fm.m[0]));
   }
   q.n += __popc(who);
 }
 
 // A leaf opened by the rays of `om`: its particles as point masses, with their
 // softening where the leaf applies it (quadTree.h:1017-1077).
-template <bool PHI, bool SCREEN, bool SHEET>
-__device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk &w, StripWarp &W, int node, int p0, int n,
-                                           unsigned om, const ExpTab &tab, StripAcc &L) {
+template <bool PHI, bool SCREEN, bool SHEET, int R>
+__device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk<R> &w, StripWarp &W, int node, int p0,
+                                           int n, const StripMask<R> &om, const ExpTab &tab, StripAcc *LL) {
   float4 Q = make_float4(0.f, 0.f, 0.f, 0.f);
   if (w.lane < n) Q = __ldg(T.parts + p0 + w.lane);  // in flight with the node's row
   const GNode *nd = T.nodes + node;
   const double width = nd->width;
-  const bool mine = om >> w.lane & 1u;
-  const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
-  const bool nearc = mine && (cx * cx + cy * cy < nd->near2);
+  unsigned nearc = 0;  // bit r: this lane's r-th ray is within the near radius
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const double cx = nd->cx - w.rx[r], cy = nd->cy - w.ry[r];
+    if (w.has(om.m, r) && cx * cx + cy * cy < nd->near2) nearc |= 1u << r;
+  }
   const double s2 = T.s2, pia = T.pia;
   // A particle within the 1e-10 of the coincidence clamp lies in a leaf whose
   // near radius (2.41 widths) the ray is in, unless the leaf is narrower than
   // that; other leaves need neither the clamp nor the softening test.
-  const bool plain = !__any_sync(kFull, nearc) && width > 1e-9 && om == w.vmask;
+  const bool plain = !__any_sync(kFull, nearc != 0u) && width > 1e-9 && om.is(w.vmask);
   for (int q0 = 0; q0 < n; q0 += 32) {
     const int m = min(32, n - q0);
     __syncwarp();
@@ -261,68 +298,85 @@ __device__ __forceinline__ void strip_leaf(const StripTree &T, const StripWalk &
       for (int j = 0; j < m; ++j, row += 2) {
         const double2 c = row[0];
         const double mpi = row[1].x;
-        const double x0 = c.x - w.rx, x1 = c.y - w.ry;
-        const double xx = __dmul_rn(x0, x0), rr = __fma_rn(x1, x1, xx);
-        const double ir2 = strip_rcp(rr);
-        double pre = __dmul_rn(mpi, ir2);
-        if (SCREEN) pre = __dmul_rn(pre, strip_exp_neg(__dmul_rn(rr, s2), tab));  // mass scr / (pi r^2)
-        const double gc = __dmul_rn(pre, ir2), t = SHEET ? __fma_rn(-pia, mpi, pre) : pre;
-        L.a0 = __fma_rn(-t, x0, L.a0);
-        L.a1 = __fma_rn(-t, x1, L.a1);
-        L.g0 = __fma_rn(-gc, __fma_rn(-x1, x1, xx), L.g0);
-        L.g1 = __fma_rn(-gc, __dmul_rn(x0, x1), L.g1);
-        if (PHI) L.p += 0.5 * pre * rr * log(rr) - 0.5 * pia * mpi * rr;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          StripAcc &L = LL[r];
+          const double x0 = c.x - w.rx[r], x1 = c.y - w.ry[r];
+          const double xx = __dmul_rn(x0, x0), rr = __fma_rn(x1, x1, xx);
+          const double ir2 = strip_rcp(rr);
+          double pre = __dmul_rn(mpi, ir2);
+          if (SCREEN) pre = __dmul_rn(pre, strip_exp_neg(__dmul_rn(rr, s2), tab));  // mass scr / (pi r^2)
+          const double gc = __dmul_rn(pre, ir2), t = SHEET ? __fma_rn(-pia, mpi, pre) : pre;
+          L.a0 = __fma_rn(-t, x0, L.a0);
+          L.a1 = __fma_rn(-t, x1, L.a1);
+          L.g0 = __fma_rn(-gc, __fma_rn(-x1, x1, xx), L.g0);
+          L.g1 = __fma_rn(-gc, __dmul_rn(x0, x1), L.g1);
+          if (PHI) L.p += 0.5 * pre * rr * log(rr) - 0.5 * pia * mpi * rr;
+        }
       }
     } else {
 #pragma unroll 1
       for (int j = 0; j < m; ++j, row += 2) {
         const double2 c = row[0], ms = row[1];
-        const double x0 = c.x - w.rx, x1 = c.y - w.ry;
-        const double xx = __dmul_rn(x0, x0);
-        double rr = __fma_rn(x1, x1, xx);
-        const double t2 = __dmul_rn(rr, s2);
-        rr = rr < 1e-20 ? 1e-20 : rr;
-        const double ir2 = strip_rcp(rr);
-        double pre = __dmul_rn(ms.x, ir2);
-        if (SCREEN) pre = __dmul_rn(pre, strip_exp_neg(t2, tab));
-        const double gc = __dmul_rn(pre, ir2), t = SHEET ? __fma_rn(-pia, ms.x, pre) : pre;
-        if (mine) {
-          L.a0 = __fma_rn(-t, x0, L.a0);
-          L.a1 = __fma_rn(-t, x1, L.a1);
-          L.g0 = __fma_rn(-gc, __fma_rn(-x1, x1, xx), L.g0);
-          L.g1 = __fma_rn(-gc, __dmul_rn(x0, x1), L.g1);
-          if (PHI) L.p += 0.5 * pre * rr * log(rr) - 0.5 * pia * ms.x * rr;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          StripAcc &L = LL[r];
+          const double x0 = c.x - w.rx[r], x1 = c.y - w.ry[r];
+          const double xx = __dmul_rn(x0, x0);
+          double rr = __fma_rn(x1, x1, xx);
+          const double t2 = __dmul_rn(rr, s2);
+          rr = rr < 1e-20 ? 1e-20 : rr;
+          const double ir2 = strip_rcp(rr);
+          double pre = __dmul_rn(ms.x, ir2);
+          if (SCREEN) pre = __dmul_rn(pre, strip_exp_neg(t2, tab));
+          const double gc = __dmul_rn(pre, ir2), t = SHEET ? __fma_rn(-pia, ms.x, pre) : pre;
+          if (w.has(om.m, r)) {
+            L.a0 = __fma_rn(-t, x0, L.a0);
+            L.a1 = __fma_rn(-t, x1, L.a1);
+            L.g0 = __fma_rn(-gc, __fma_rn(-x1, x1, xx), L.g0);
+            L.g1 = __fma_rn(-gc, __dmul_rn(x0, x1), L.g1);
+            if (PHI) L.p += 0.5 * pre * rr * log(rr) - 0.5 * pia * ms.x * rr;
+          }
+          if ((nearc >> r & 1u) && rr < ms.y) strip_soften<PHI>(T.dev, x0, x1, rr, __ldg(T.parts + p0 + q0 + j), L);
         }
-        if (nearc && rr < ms.y) strip_soften<PHI>(T.dev, x0, x1, rr, __ldg(T.parts + p0 + q0 + j), L);
       }
     }
   }
 }
 
 // Softened particles listed at an internal node (quadTree.h:1048-1077).
-template <bool PHI>
-__device__ __forceinline__ void strip_bigs(const StripTree &T, const StripWalk &w, int node, unsigned om, StripAcc &L) {
+template <bool PHI, int R>
+__device__ __forceinline__ void strip_bigs(const StripTree &T, const StripWalk<R> &w, int node, const StripMask<R> &om,
+                                           StripAcc *LL) {
   const GNode *nd = T.nodes + node;
-  const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
-  if (!((om >> w.lane & 1u) && cx * cx + cy * cy < nd->near2)) return;
 #pragma unroll 1
-  for (int b = nd->bstart, e = b + nd->bcount; b < e; ++b) {
-    const float4 Q = __ldg(T.dev->bigs + b);
-    const double x0 = (double)Q.x - w.rx, x1 = (double)Q.y - w.ry;
-    double rr = x0 * x0 + x1 * x1;
-    if (rr < 1e-20) rr = 1e-20;
-    const double size = (double)Q.w;
-    if (rr < 4 * size * size) strip_soften<PHI>(T.dev, x0, x1, rr, Q, L);
+  for (int r = 0; r < R; ++r) {
+    const double rx = r == 0 ? w.rx[0] : w.rx[R - 1], ry = r == 0 ? w.ry[0] : w.ry[R - 1];
+    const double cx = nd->cx - rx, cy = nd->cy - ry;
+    if (!((r == 0 ? om.m[0] : om.m[R - 1]) >> w.lane & 1u) || !(cx * cx + cy * cy < nd->near2)) continue;
+#pragma unroll 1
+    for (int b = nd->bstart, e = b + nd->bcount; b < e; ++b) {
+      const float4 Q = __ldg(T.dev->bigs + b);
+      const double x0 = (double)Q.x - rx, x1 = (double)Q.y - ry;
+      double rr = x0 * x0 + x1 * x1;
+      if (rr < 1e-20) rr = 1e-20;
+      const double size = (double)Q.w;
+      if (rr < 4 * size * size) {
+        if (r == 0)
+          strip_soften<PHI>(T.dev, x0, x1, rr, Q, LL[0]);
+        else
+          strip_soften<PHI>(T.dev, x0, x1, rr, Q, LL[R - 1]);
+      }
+    }
   }
 }
 
 // The walk's nodes in [base, end): base moves to the next node to visit (it
 // may pass end), resume is this lane's next node (it sits out nodes before
 // it).  The loop keeps one copy of each evaluation, for the instruction cache.
-template <bool PHI, bool SCREEN, bool SHEET>
-__device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk &w, StripWarp &W, const ExpTab &tab,
-                                            int &base, int end, int &resume, StripAcc &L) {
-  const bool mine = w.vmask >> w.lane & 1u;
+template <bool PHI, bool SCREEN, bool SHEET, int R>
+__device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk<R> &w, StripWarp &W, const ExpTab &tab,
+                                            int &base, int end, int *resume, StripAcc *L) {
   StripQueue q;
   while (base < end) {
     const int sbase = base, i = base + w.lane;
@@ -358,35 +412,50 @@ __device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk 
     const unsigned ev = mm | __ballot_sync(kFull, live && cls == 2 && info != 0);
     int next = max(min(base + 32, end), (int)__reduce_max_sync(kFull, isA ? (unsigned)skip : 0u));
     // slow: node by node, some rays sit out part of the strip or take a test
-    const bool slow = mm != 0u || __any_sync(kFull, mine && resume > base);
-    unsigned todo = slow ? am | ev : ev, pend = slow ? 0u : am, fm = w.vmask;
+    bool late = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) late = late || (w.has(w.vmask, r) && resume[r] > base);
+    const bool slow = mm != 0u || __any_sync(kFull, late);
+    unsigned todo = slow ? am | ev : ev, pend = slow ? 0u : am;
+    StripMask<R> fm;
+#pragma unroll
+    for (int r = 0; r < R; ++r) fm.m[r] = w.vmask[r];
     for (;;) {
       // the next node with particles to evaluate, and the far-field rows before it
       int node = -1, inf = 0;
-      unsigned om = w.vmask, push = pend;
+      unsigned push = pend;
+      StripMask<R> om;
+#pragma unroll
+      for (int r = 0; r < R; ++r) om.m[r] = w.vmask[r];
       while (todo) {
         const int b = __ffs(todo) - 1;
         todo &= todo - 1;
         inf = __shfl_sync(kFull, info, b);
         if (slow) {
-          const unsigned act = __ballot_sync(kFull, mine && base + b >= resume);
+          StripMask<R> act;
+#pragma unroll
+          for (int r = 0; r < R; ++r) act.m[r] = __ballot_sync(kFull, base + b >= resume[r]) & w.vmask[r];
           if (am >> b & 1u) {
             if (w.lane == b) fm = act;
-            if (act) pend |= 1u << b;
+            if (act.any()) pend |= 1u << b;
             continue;
           }
           const int sk = __shfl_sync(kFull, skip, b);
           om = act;
           if (mm >> b & 1u) {
             const GNode *nd = T.nodes + base + b;
-            const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
-            om = __ballot_sync(kFull, cx * cx + cy * cy < nd->open2) & act;
-            const unsigned fa = act & ~om;
+            StripMask<R> fa;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const double cx = nd->cx - w.rx[r], cy = nd->cy - w.ry[r];
+              om.m[r] = __ballot_sync(kFull, cx * cx + cy * cy < nd->open2) & act.m[r];
+              fa.m[r] = act.m[r] & ~om.m[r];
+              if (w.has(fa.m, r)) resume[r] = sk;
+            }
             if (w.lane == b) fm = fa;
-            if (fa) pend |= 1u << b;
-            if (fa >> w.lane & 1u) resume = sk;
+            if (fa.any()) pend |= 1u << b;
           }
-          if (om == 0u) {  // nobody opens it: past its subtree
+          if (!om.any()) {  // nobody opens it: past its subtree
             todo &= sk - base >= 32 ? 0u : ~((1u << (sk - base)) - 1u);
             next = max(next, sk);
             continue;
@@ -400,63 +469,78 @@ __device__ __forceinline__ void strip_range(const StripTree &T, const StripWalk 
       }
       if (slow) {
         push = pend;
-        q.masked = q.masked || __any_sync(kFull, (push >> w.lane & 1u) && fm != w.vmask);
+        q.masked = q.masked || __any_sync(kFull, (push >> w.lane & 1u) && !fm.is(w.vmask));
       }
       strip_push(w, W, q, push, r0, r1, q2, fm);
       pend &= ~push;
       bool flush = q.n > 0;
       if (node < 0) {
-        base = slow ? max(next, (int)__reduce_min_sync(kFull, mine ? (unsigned)resume : 0x7fffffffu)) : next;
+        base = next;
+        if (slow) {
+          unsigned first = 0x7fffffffu;
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (w.has(w.vmask, r)) first = min(first, (unsigned)resume[r]);
+          base = max(base, (int)__reduce_min_sync(kFull, first));
+        }
         flush = q.n >= 32 || (base >= end && q.n > 0);
       }
       if (flush) {
         __syncwarp();
         if (q.masked)
-          strip_far_rows<PHI, SCREEN, SHEET, true>(T, w, W, q.n, tab, L);
+          strip_far_rows<PHI, SCREEN, SHEET, true, R>(T, w, W, q.n, tab, L);
         else
-          strip_far_rows<PHI, SCREEN, SHEET, false>(T, w, W, q.n, tab, L);
+          strip_far_rows<PHI, SCREEN, SHEET, false, R>(T, w, W, q.n, tab, L);
         __syncwarp();
         q.n = 0;
         q.masked = false;
       }
       if (node < 0) break;
       if (inf < 0)
-        strip_leaf<PHI, SCREEN, SHEET>(T, w, W, node, __shfl_sync(kFull, pstart, node - sbase), -inf, om, tab, L);
+        strip_leaf<PHI, SCREEN, SHEET, R>(T, w, W, node, __shfl_sync(kFull, pstart, node - sbase), -inf, om, tab, L);
       else
-        strip_bigs<PHI>(T, w, node, om, L);
+        strip_bigs<PHI, R>(T, w, node, om, L);
     }
   }
 }
 
-template <bool PHI>
-__device__ __forceinline__ void strip_run(const StripTree &T, const StripWalk &w, StripWarp &W, const ExpTab &tab,
-                                          int base, int end, int resume, StripAcc &L) {
+template <bool PHI, int R>
+__device__ __forceinline__ void strip_run(const StripTree &T, const StripWalk<R> &w, StripWarp &W, const ExpTab &tab,
+                                          int base, int end, int *resume, StripAcc *L) {
   if (T.pia != 0.0)
-    strip_range<PHI, true, true>(T, w, W, tab, base, end, resume, L);
+    strip_range<PHI, true, true, R>(T, w, W, tab, base, end, resume, L);
   else if (T.s2 != 0.0)
-    strip_range<PHI, true, false>(T, w, W, tab, base, end, resume, L);
+    strip_range<PHI, true, false, R>(T, w, W, tab, base, end, resume, L);
   else
-    strip_range<PHI, false, false>(T, w, W, tab, base, end, resume, L);
+    strip_range<PHI, false, false, R>(T, w, W, tab, base, end, resume, L);
 }
 
-// One whole walk for the ray (rx, ry), added to acc[c * A], c = 0..4 (and 5,
-// PHI) = {alpha0, alpha1, kappa, gamma0, gamma1, phi}.
-template <bool PHI>
-__device__ __forceinline__ void walk_strip(const TreeDev &D, double rx, double ry, bool valid, StripWarp &W,
-                                           const ExpTab &tab, double *acc, int A) {
+// One whole walk for the R rays (rx[r], ry[r]) of every lane, added to
+// acc[(6 r + c) * A], c = 0..4 (and 5, PHI) = {alpha0, alpha1, kappa, gamma0,
+// gamma1, phi}.
+template <bool PHI, int R>
+__device__ __forceinline__ void walk_strip(const TreeDev &D, const double *rx, const double *ry, const bool *valid,
+                                           StripWarp &W, const ExpTab &tab, double *acc, int A) {
   const int nn = D.nnodes;
   if (nn == 0) return;
   const StripTree T(D);
-  const StripWalk w = strip_begin(rx, ry, valid);
-  StripAcc L;
-  strip_run<PHI>(T, w, W, tab, 0, nn, valid ? 0 : 0x7fffffff, L);
-  acc[0] += L.a0;
-  acc[A] += L.a1;
-  acc[2 * A] += L.k;
-  acc[3 * A] += L.g0;
-  acc[4 * A] += 2.0 * L.g1;
-  if (PHI) acc[5 * A] += L.p;
-  if (D.inv_area != 0.0 && valid) acc[2 * A] -= D.inv_area * D.root_mass;  // every mass enters a walk once
+  const StripWalk<R> w = strip_begin<R>(rx, ry, valid);
+  StripAcc L[R];
+  int resume[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) resume[r] = valid[r] ? 0 : 0x7fffffff;
+  strip_run<PHI, R>(T, w, W, tab, 0, nn, resume, L);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    double *o = acc + 6 * r * A;
+    o[0] += L[r].a0;
+    o[A] += L[r].a1;
+    o[2 * A] += L[r].k;
+    o[3 * A] += L[r].g0;
+    o[4 * A] += 2.0 * L[r].g1;
+    if (PHI) o[5 * A] += L[r].p;
+    if (D.inv_area != 0.0 && w.has(w.vmask, r)) o[2 * A] -= D.inv_area * D.root_mass;  // every mass enters a walk once
+  }
 }
 
 // The part [s0, end) of a walk shared by several warps (s0 a multiple of
@@ -468,7 +552,7 @@ template <bool PHI>
 __device__ __forceinline__ bool walk_strip_part(const TreeDev &D, double rx, double ry, bool valid, StripWarp &W,
                                                     const ExpTab &tab, int s0, int end, StripAcc &L) {
   const StripTree T(D);
-  const StripWalk w = strip_begin(rx, ry, valid);
+  const StripWalk<1> w = strip_begin<1>(&rx, &ry, &valid);
   int resume = valid ? s0 : 0x7fffffff;
   const int a = __ldg(D.cutanc + (size_t)kMaxDepth * (s0 / kCutStep) + w.lane);
   int skip = 0, cls = 2;
@@ -485,13 +569,13 @@ __device__ __forceinline__ bool walk_strip_part(const TreeDev &D, double rx, dou
     todo &= todo - 1;
     const int node = __shfl_sync(kFull, a, b), sk = __shfl_sync(kFull, skip, b), c = __shfl_sync(kFull, cls, b);
     const GNode *nd = T.nodes + node;
-    const double cx = nd->cx - w.rx, cy = nd->cy - w.ry;
+    const double cx = nd->cx - rx, cy = nd->cy - ry;
     // every ancestor's subtree holds s0, so the outermost one not opened decides
     if (c == 1 || !(cx * cx + cy * cy < nd->open2)) resume = max(resume, sk);
   }
   const int base = (int)__reduce_min_sync(kFull, valid ? (unsigned)resume : 0x7fffffffu);
   if (base >= end) return false;
-  strip_run<PHI>(T, w, W, tab, base, end, resume, L);
+  strip_run<PHI, 1>(T, w, W, tab, base, end, &resume, &L);
   return true;
 }
 

@@ -107,3 +107,18 @@ def test_small_lens_calls_match_large_ones(n):
         ys, As = lens.rayshooterInternal(x[:n], None if z is None else z[:n])
         assert np.abs(ys - y[:n]).max() < 1e-11 * np.abs(y).max()
         assert np.abs(As - A[:n]).max() < 1e-8 * np.abs(A).max()
+
+
+def test_two_rays_per_lane_match_one():
+    """Grids whose ray counts take the two-ray kernel (131,044 rays: one wave of
+    it) and the one-ray kernel (their first 66,049 rays) agree bit for bit."""
+    spec = synth.light_cone(seed=12, n_total=40000, n_planes=2, halos_per_plane=4)
+    lens = glb.lens_from_spec(spec)
+    x = synth.grid_positions(362, range_rad=40 * synth.ARCSEC)
+    y, A = lens.rayshooterInternal(x)
+    ys, As = lens.rayshooterInternal(x[:66049])
+    assert np.array_equal(y[:66049], ys) and np.array_equal(A[:66049], As)
+    zs = np.random.default_rng(3).uniform(0.05, 3.0, len(x))
+    y, A = lens.rayshooterInternal(x, zs)
+    ys, As = lens.rayshooterInternal(x[:66049], zs[:66049])
+    assert np.array_equal(y[:66049], ys) and np.array_equal(A[:66049], As)
