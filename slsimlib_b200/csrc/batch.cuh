@@ -70,10 +70,11 @@ const ExpTab *batch_exptab(const std::vector<glb_lens *> &lenses) {
         if (h->tree && h->tree->dev.exptab) return h->tree->dev.exptab;
   return nullptr;
 }
-// The strip form adds the strip walk's: a StripWarp per warp and the
-// exponential's table.
+// The split form adds the list walk's (a ListWarp per warp), the strip form
+// the strip walk's (a StripWarp per warp and the exponential's table).
 inline size_t batch_smem_bytes(int block, int form) {
   size_t b = (size_t)kBatchSmemDoubles * block * sizeof(double);
+  if (form == GLB_PREC_SPLIT) b += (size_t)(block / 32) * sizeof(ListWarp);
   if (form == kStripForm)
     b += (size_t)(block / 32) * sizeof(StripWarp) + sizeof(ExpTab);
   return b;
@@ -85,7 +86,7 @@ inline size_t batch_smem_bytes(int block, int form) {
 template <int PREC>
 __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *halos, const NFWTables *tab,
                                             double xx0, double xx1, bool valid, double *f, double *h,
-                                            int stride, StripWarp *W, const ExpTab *etab) {
+                                            int stride, StripWarp *W, const ExpTab *etab, ListWarp *Lw) {
   for (int c = 0; c < 5; ++c) f[c * stride] = 0.0;
   for (int k = 0; k < P.nhalo; ++k) {
     const HaloDev *H = halos + P.halo0 + k;
@@ -95,8 +96,10 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
       for (int c = 0; c < 5; ++c) h[c] = 0.0;
       if constexpr (PREC == kStripForm)
         particle_halo_f64<false>(H->tree, xc0, xc1, valid, *W, *etab, h, 1);
+      else if constexpr (PREC == GLB_PREC_SPLIT)
+        particle_halo_list(H->tree, xc0, xc1, valid, *Lw, h);
       else
-        particle_halo_acc<PREC, false, true>(H->tree, xc0, xc1, valid, h);
+        particle_halo_acc<PREC>(H->tree, xc0, xc1, valid, h);
       // force_halo negates the walk's alpha (particle_halo.h:432-433)
       a[0] = -h[0];
       a[1] = -h[1];
@@ -128,9 +131,9 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
   }
 }
 template <int PREC>
-// capped at 80 registers (3 blocks of 256 per SM) for occupancy (64 registers measured slower here);
+// 128 registers (2 blocks of 256 per SM): 48 uneven lenses, list walk 72.9 ms; 80 registers 90.0, 64 registers 113
 // dynamic shared memory: batch_smem_bytes(blockDim.x)
-__global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
+__global__ void __launch_bounds__(256, 2) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
                                                NFWTables tab, const double *xs, const unsigned *outidx,
                                                double *y, double *A, int *counter, const ExpTab *exptab) {
   extern __shared__ __align__(16) double bsm[];
@@ -141,6 +144,9 @@ __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchun
   double *h = bsm + 17 * B + 5 * threadIdx.x;  // h[0..4]
   StripWarp *W = nullptr;
   ExpTab *etab = nullptr;
+  ListWarp *Lw = nullptr;
+  if constexpr (PREC == GLB_PREC_SPLIT)
+    Lw = reinterpret_cast<ListWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
   if constexpr (PREC == kStripForm) {
     W = reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
     etab = reinterpret_cast<ExpTab *>(reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + B / 32);
@@ -204,7 +210,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const Chunk *chunks, int nchun
       const bool v = valid && j < jmax;
       {
         const PlaneDev &P = L.planes[j];
-        plane_force<PREC>(P, L.halos, &tab, st[0] * P.Dphys, st[B] * P.Dphys, v, f, h, B, W, etab);
+        plane_force<PREC>(P, L.halos, &tab, st[0] * P.Dphys, st[B] * P.Dphys, v, f, h, B, W, etab, Lw);
       }
       if (v) {
         // include/lens.h:1027-1066, the state reloaded from shared memory
@@ -290,7 +296,7 @@ int persistent_grid(int block, int form, int *grid) {
   const void *k = form == GLB_PREC_SPLIT ? (const void *)k_batch<GLB_PREC_SPLIT>
                   : form == kStripForm   ? (const void *)k_batch<kStripForm>
                                          : (const void *)k_batch<GLB_PREC_FP64>;
-  if (form == kStripForm)  // more than the default 48 KB
+  if (form != GLB_PREC_FP64)  // more than the default 48 KB
     CKR(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes(256, form)));
   CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, batch_smem_bytes(block, form)));
   *grid = sms * std::max(per_sm, 1);

@@ -122,3 +122,30 @@ def test_two_rays_per_lane_match_one():
     y, A = lens.rayshooterInternal(x, zs)
     ys, As = lens.rayshooterInternal(x[:66049], zs[:66049])
     assert np.array_equal(y[:66049], ys) and np.array_equal(A[:66049], As)
+
+
+@pytest.mark.parametrize("n,size,sign,inv_area", [
+    (1, 0.01, False, 0.0), (2, 0.01, False, 0.0), (21, 0.5, False, 0.0), (700, 0.02, True, 0.3),
+    (3000, 0.3, False, 0.2), (60000, 0.001, False, 0.0), (200000, 0.0005, False, 0.0),
+])
+@pytest.mark.parametrize("side", [1, 5, 33, 96])
+def test_list_walk_matches_the_walk_of_each_ray(n, size, sign, inv_area, side):
+    """The batch's split form (list walk) against the lens path of a plane with
+    two particle haloes (a walk per ray): the same FP32 blocks in the same
+    order, so only the FP64 recursion may round differently."""
+    p, q = _cluster(n + 1, n, size, sign), _cluster(n + 2, 40, 0.05)
+    for c in (p, q):
+        c["Mass"] *= 1e10
+    lens = glb.Lens(2.0)
+    lens.insertMainHalo(glb.LensHaloParticles(p, 0.3, inv_area=inv_area), True)
+    lens.insertMainHalo(glb.LensHaloParticles(q, 0.3), True)
+    assert lens.getNplanes() == 1
+    rng = 100 * synth.ARCSEC
+    b = glb.GridBatch([lens], [side], [(0.0, 0.0)], [rng], glb.PREC_SPLIT)
+    for block in (64, 128, 256):
+        b.set_block(block)
+        b.run()
+        y, A = b.result(0)
+        g = glb.GridMap(lens, side, (0.0, 0.0), rng, glb.PREC_SPLIT)
+        assert np.abs(y - g.y).max() <= 1e-13 * np.abs(g.y).max()
+        assert np.abs(A - g.A).max() <= 1e-13 * np.abs(g.A).max()
