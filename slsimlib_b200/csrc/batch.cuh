@@ -52,15 +52,25 @@ struct Chunk {
 // distinct banks).  Keeping them out of registers leaves the tree walk the
 // registers it needs.
 constexpr int kBatchSmemDoubles = 22;
-// The kernel's form: GLB_PREC_SPLIT, GLB_PREC_FP64 (the node-at-a-time walk:
-// batches with NFW haloes, see launch_plane_steps) or kStripForm (the strip
-// walk: every other FP64 batch).
-constexpr int kStripForm = 3;
+// The kernel's form.  FP64: GLB_PREC_FP64 (the node-at-a-time walk: batches with
+// NFW haloes, see launch_plane_steps) or kStripForm (the strip walk: every other
+// batch).  Split: kListForm (the list walk) or, for batches with a tree of more
+// than kListMaxNodes nodes, GLB_PREC_SPLIT (the node-at-a-time walk): where a
+// warp's rays are spread over several leaves, most cells near the opening radius
+// are mixed.  One plane, 512^2 rays over 30 arcsec, node by node / list, ms: 2^16
+// particles 6.5 / 3.8, 2^18 7.8 / 4.8, 2^20 (151,000 nodes) 9.9 / 9.1, 2^22
+// (604,000) 16.7 / 22.1; over 600 arcsec 2^20 18.9 / 17.7, 2^22 62.5 / 59.2.
+constexpr int kStripForm = 3, kListForm = 4;
+constexpr int kListMaxNodes = 200000;
 int batch_form(const std::vector<glb_lens *> &lenses, int precision) {
-  if (precision == GLB_PREC_SPLIT) return precision;
-  for (const glb_lens *l : lenses)
-    if (l->has_nfw) return GLB_PREC_FP64;
-  return kStripForm;
+  for (const glb_lens *l : lenses) {
+    if (precision == GLB_PREC_FP64 && l->has_nfw) return GLB_PREC_FP64;
+    if (precision == GLB_PREC_SPLIT)
+      for (const PlaneHost *p : l->planes)
+        for (const glb_halo *h : p->halos)
+          if (h->tree && h->tree->dev.nnodes > kListMaxNodes) return GLB_PREC_SPLIT;
+  }
+  return precision == GLB_PREC_SPLIT ? kListForm : kStripForm;
 }
 // The exponential's tables: those of any particle tree in the batch.
 const ExpTab *batch_exptab(const std::vector<glb_lens *> &lenses) {
@@ -70,11 +80,11 @@ const ExpTab *batch_exptab(const std::vector<glb_lens *> &lenses) {
         if (h->tree && h->tree->dev.exptab) return h->tree->dev.exptab;
   return nullptr;
 }
-// The split form adds the list walk's (a ListWarp per warp), the strip form
+// The list form adds a ListWarp per warp, the strip form
 // the strip walk's (a StripWarp per warp and the exponential's table).
 inline size_t batch_smem_bytes(int block, int form) {
   size_t b = (size_t)kBatchSmemDoubles * block * sizeof(double);
-  if (form == GLB_PREC_SPLIT) b += (size_t)(block / 32) * sizeof(ListWarp);
+  if (form == kListForm) b += (size_t)(block / 32) * sizeof(ListWarp);
   if (form == kStripForm)
     b += (size_t)(block / 32) * sizeof(StripWarp) + sizeof(ExpTab);
   return b;
@@ -96,10 +106,10 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
       for (int c = 0; c < 5; ++c) h[c] = 0.0;
       if constexpr (PREC == kStripForm)
         particle_halo_f64<false>(H->tree, xc0, xc1, valid, *W, *etab, h, 1);
-      else if constexpr (PREC == GLB_PREC_SPLIT)
+      else if constexpr (PREC == kListForm)
         particle_halo_list(H->tree, xc0, xc1, valid, *Lw, h);
       else
-        particle_halo_acc<PREC>(H->tree, xc0, xc1, valid, h);
+        particle_halo_acc<PREC, false, true>(H->tree, xc0, xc1, valid, h);
       // force_halo negates the walk's alpha (particle_halo.h:432-433)
       a[0] = -h[0];
       a[1] = -h[1];
@@ -131,9 +141,11 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
   }
 }
 template <int PREC>
-// 128 registers (2 blocks of 256 per SM): 48 uneven lenses, list walk 72.9 ms; 80 registers 90.0, 64 registers 113
+// The list and strip forms take 128 registers (2 blocks of 256 per SM): 48 uneven
+// lenses, list form, 70.3 ms; with 80 registers 90.  The node-at-a-time forms take
+// 80, for occupancy (64 registers measured slower there).
 // dynamic shared memory: batch_smem_bytes(blockDim.x)
-__global__ void __launch_bounds__(256, 2) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
+__global__ void __launch_bounds__(256, PREC == kListForm || PREC == kStripForm ? 2 : 3) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,
                                                NFWTables tab, const double *xs, const unsigned *outidx,
                                                double *y, double *A, int *counter, const ExpTab *exptab) {
   extern __shared__ __align__(16) double bsm[];
@@ -145,7 +157,7 @@ __global__ void __launch_bounds__(256, 2) k_batch(const Chunk *chunks, int nchun
   StripWarp *W = nullptr;
   ExpTab *etab = nullptr;
   ListWarp *Lw = nullptr;
-  if constexpr (PREC == GLB_PREC_SPLIT)
+  if constexpr (PREC == kListForm)
     Lw = reinterpret_cast<ListWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
   if constexpr (PREC == kStripForm) {
     W = reinterpret_cast<StripWarp *>(bsm + kBatchSmemDoubles * B) + (threadIdx.x >> 5);
@@ -294,9 +306,10 @@ int persistent_grid(int block, int form, int *grid) {
   CKR(cudaGetDevice(&dev));
   CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const void *k = form == GLB_PREC_SPLIT ? (const void *)k_batch<GLB_PREC_SPLIT>
+                  : form == kListForm    ? (const void *)k_batch<kListForm>
                   : form == kStripForm   ? (const void *)k_batch<kStripForm>
                                          : (const void *)k_batch<GLB_PREC_FP64>;
-  if (form != GLB_PREC_FP64)  // more than the default 48 KB
+  if (form == kListForm || form == kStripForm)  // more than the default 48 KB
     CKR(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes(256, form)));
   CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, batch_smem_bytes(block, form)));
   *grid = sms * std::max(per_sm, 1);
@@ -309,6 +322,8 @@ int launch_batch(int form, int grid, int block, cudaStream_t s, const Chunk *chu
   const size_t smem = batch_smem_bytes(block, form);
   if (form == GLB_PREC_SPLIT)
     k_batch<GLB_PREC_SPLIT><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
+  else if (form == kListForm)
+    k_batch<kListForm><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
   else if (form == kStripForm)
     k_batch<kStripForm><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
   else

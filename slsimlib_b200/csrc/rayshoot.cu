@@ -414,7 +414,7 @@ __global__ void k_grid(size_t N1d, double c0, double c1, double range, double *x
 
 // A particle halo's tree force at (rx, ry), periodic images included; FP64 here
 // is the node-at-a-time walk (particle_halo_f64 is the strip walk).
-template <int PREC, bool COUNT = false, bool MERGE = true>
+template <int PREC, bool COUNT = false, bool SKIPNEAR = false, bool MERGE = true>
 __device__ __forceinline__ void particle_halo_acc(const TreeDev &T, double rx, double ry, bool valid, double *acc,
                                                   WalkCount *wc = nullptr) {
   auto walk = [&](double x, double y) {
@@ -423,7 +423,7 @@ __device__ __forceinline__ void particle_halo_acc(const TreeDev &T, double rx, d
     else if (PREC == GLB_PREC_FP32)
       walk_split<true>(T, x, y, valid, acc);
     else
-      walk_split<false, MERGE>(T, x, y, valid, acc);
+      walk_split<false, SKIPNEAR, MERGE>(T, x, y, valid, acc);
   };
   if (T.periodic) {
     // force2D_recur with a periodic buffer: nine shifted copies (quadTree.h:944-974)
@@ -1055,7 +1055,7 @@ __device__ __forceinline__ void tree_force(const TreeDev &T, size_t n, const dou
     x1 = x[2 * k + 1];
   }
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  particle_halo_acc<PREC, false, false>(T, x0, x1, valid, acc);  // a flush per opened leaf
+  particle_halo_acc<PREC, false, false, false>(T, x0, x1, valid, acc);  // a flush per opened leaf
   if (!valid) return;
   for (int c = 0; c < 5; ++c) out[5 * k + c] = acc[c];
 }

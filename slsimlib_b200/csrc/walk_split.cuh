@@ -204,11 +204,15 @@ __device__ __forceinline__ void bspline_f32(float x0, float x1, float r, float M
 // from FP32 coordinates, FP32 opening tests and sums throughout, the
 // reference's FP32-evaluated B-spline; it keeps no FP64 arithmetic and so no
 // guarantee of the FP64 form's interaction set or precision.
+// SKIPNEAR: take the near-field test only where it is read (leaves, internal
+// nodes with big particles).  Same results; it pays in the batched kernel
+// (+1.1 % on 256 uneven lenses) but makes the one-ray plane step spill far
+// more (45M -> 27M rays/s on a 512^2 single plane), so only k_batch sets it.
 // MERGE: far leaves join the running partial sums (below); without it every
 // opened leaf is summed on its own, flushed before and after (the one-ray
 // tree-force kernel: merging made it spill 232 / 420 B against 76 / 192 B and
 // run 9 % slower at opening angle 0.3).
-template <bool PURE = false, bool MERGE = true>
+template <bool PURE = false, bool SKIPNEAR = false, bool MERGE = true>
 __device__ __forceinline__ void walk_split(const TreeDev &T, double rx, double ry, bool valid, double *acc) {
   const bool screen = T.screen2 != 0.0;
   const float s2f = (float)T.screen2;
@@ -272,7 +276,7 @@ __device__ __forceinline__ void walk_split(const TreeDev &T, double rx, double r
       continue;
     }
     bool nearc = false;
-    if (open) {
+    if (open && (!SKIPNEAR || c3.y || c3.w > 0)) {
       const float e = r2f - c1.y;
       nearc = e < 0.f;
       if (!PURE && fabsf(e) <= kAmbiguous * c1.y) nearc = node_test_f64(T.nodes + node, rx, ry, 1);
@@ -360,7 +364,7 @@ __device__ __forceinline__ void walk_split(const TreeDev &T, double rx, double r
       }
       node = skip;
     } else {
-      if (__any_sync(kFull, nearc)) {
+      if ((!SKIPNEAR || c3.w > 0) && __any_sync(kFull, nearc)) {
         const int b0 = c3.z, b1 = b0 + c3.w;
         for (int b = b0; b < b1; ++b) {
           const float4 P = __ldg(T.bigs + b);
@@ -452,7 +456,7 @@ __device__ __forceinline__ void leaf_term(const TreeDev &T, float4 P, int p, flo
 // walk_split<false> does for one, while the node rows, the warp vote, the
 // loop control and the leaf particles are loaded and executed once for both.
 // Each ray forms its own double-float offsets, so its terms, decisions and
-// FP64 totals are walk_split<false, false>'s: a leaf opened by a ray is
+// FP64 totals are walk_split<false, false, false>'s: a leaf opened by a ray is
 // summed on its own, flushed before and after, and the results are
 // bit-identical to the one-ray walk's.  rxy: {rx0, ry0, rx1, ry1} (the rays'
 // FP64 positions); acc0 / acc1: the rays' FP64 totals.

@@ -127,6 +127,7 @@ def test_two_rays_per_lane_match_one():
 @pytest.mark.parametrize("n,size,sign,inv_area", [
     (1, 0.01, False, 0.0), (2, 0.01, False, 0.0), (21, 0.5, False, 0.0), (700, 0.02, True, 0.3),
     (3000, 0.3, False, 0.2), (60000, 0.001, False, 0.0), (200000, 0.0005, False, 0.0),
+    (3000000, 0.0002, False, 0.0),  # more nodes than the list walk takes
 ])
 @pytest.mark.parametrize("side", [1, 5, 33, 96])
 def test_list_walk_matches_the_walk_of_each_ray(n, size, sign, inv_area, side):
