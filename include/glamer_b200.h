@@ -62,8 +62,10 @@ enum {
                          rays that share the classification of the tree's cells, so a
                          ray's result can change at the rounding level (~1e-9; the order
                          of its terms) with the other rays of its block, never its set of
-                         interactions; tree-force calls and the FP64 form are per-ray
-                         exact */
+                         interactions; tree-force calls and the FP64 form do not depend
+                         on the other rays (the FP64 form's calls below 2^16 rays, host
+                         tree forces below 2^18, add a ray's terms range by range of the
+                         tree, so that result differs by roundings from a larger call's) */
   GLB_PREC_FP32 = 2   /* plain FP32 tree walk (tree-force calls only; the precision sweep) */
 };
 

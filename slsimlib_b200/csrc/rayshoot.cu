@@ -926,9 +926,11 @@ __global__ void __launch_bounds__(32 * kSumRows) k_plane_parts_end(const __grid_
 // thread at a stride of five: a half-warp's 64-bit accesses on distinct
 // banks), and the recursion reloads theta, the plane constants and the
 // source-plane scalars after the walk.  The particle halo's terms are added
-// first, then the analytic halos' in insertion order.  Measured per 2048^2
-// light-cone step against the per-ray walks: 638 ms against 718 (two rays
-// per thread) and 771 (one); 512^2 single plane 5.56 against 5.88 ms.
+// first, then the analytic halos' in insertion order.  2048^2 light-cone step
+// 400 ms (492 with every leaf particle tested, 533 with three rows a cell and
+// the classification's dependent loads as well; 718 to 771 with a walk per
+// ray); 512^2 single plane 3.39 ms, of which far cells 0.9, leaves 0.7, mixed
+// subtrees 1.2 and the classification 0.3.
 __global__ void __launch_bounds__(128, 6) k_plane_step_split_g(const __grid_constant__ StepArgs a) {
   __shared__ double sacc[5 * 128];
   __shared__ double sxy[2 * 128];
