@@ -61,30 +61,56 @@ struct DBuf {
 cudaError_t scratch_pool(cudaMemPool_t *pool);
 
 // Scratch memory from the pool, taken and given back in the order of a stream.
+// An arena is one such allocation that later ones carve their buffers from while
+// it has room (a small tree's twenty buffers take longer to allocate than to
+// fill).
 template <typename T>
 struct ABuf {
   T *p = nullptr;
   size_t n = 0;
   cudaStream_t s;
-  explicit ABuf(cudaStream_t st) : s(st) {}
+  struct Arena *arena;
+  bool carved = false;
+  explicit ABuf(cudaStream_t st, Arena *a = nullptr) : s(st), arena(a) {}
   ABuf(const ABuf &) = delete;
   ABuf &operator=(const ABuf &) = delete;
   ~ABuf() { release(); }
   void release() {
-    if (p) cudaFreeAsync(p, s);
+    if (p && !carved) cudaFreeAsync(p, s);
     p = nullptr;
     n = 0;
+    carved = false;
   }
-  cudaError_t alloc(size_t count) {
-    release();
-    if (count == 0) return cudaSuccess;
-    cudaMemPool_t pool;
-    cudaError_t e = scratch_pool(&pool);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);
-    if (e == cudaSuccess) n = count;
-    return e;
+  cudaError_t alloc(size_t count);
+};
+struct Arena {
+  ABuf<char> mem;
+  size_t used = 0;
+  explicit Arena(cudaStream_t st) : mem(st) {}
+  char *carve(size_t bytes) {
+    const size_t at = (used + 255) / 256 * 256;
+    if (!mem.p || at + bytes > mem.n) return nullptr;
+    used = at + bytes;
+    return mem.p + at;
   }
 };
+template <typename T>
+cudaError_t ABuf<T>::alloc(size_t count) {
+  release();
+  if (count == 0) return cudaSuccess;
+  if (arena)
+    if (char *c = arena->carve(count * sizeof(T))) {
+      p = reinterpret_cast<T *>(c);
+      n = count;
+      carved = true;
+      return cudaSuccess;
+    }
+  cudaMemPool_t pool;
+  cudaError_t e = scratch_pool(&pool);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);
+  if (e == cudaSuccess) n = count;
+  return e;
+}
 
 // TreeQuadParticles built on the device.
 struct Tree {

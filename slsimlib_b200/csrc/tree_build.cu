@@ -468,9 +468,12 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   cnodes[b.pre] = c;
 }
 
-// The ancestors of every kCutStep-th node, outermost first.
-__global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc) {
+// The ancestors of every kCutStep-th node, outermost first, and the tables of
+// the strip walk's exponential.
+__global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc, ExpTab *E) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < 1024) E->lo[g] = exp(-(double)g / 1024.0);
+  if (g < 704) E->hi[g] = exp(-(double)g);
   if (g >= ncut) return;
   const int s = g * kCutStep;
   int *a = anc + (size_t)kMaxDepth * g, k = 0, node = 0;
@@ -480,12 +483,6 @@ __global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc) {
     else node = skip;
   }
   for (; k < kMaxDepth; ++k) a[k] = -1;
-}
-
-__global__ void k_exp_tables(ExpTab *E) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 1024) E->lo[i] = exp(-(double)i / 1024.0);
-  if (i < 704) E->hi[i] = exp(-(double)i);
 }
 
 __global__ void k_gather_parts(const glb_particle_rec *p, const unsigned *sidx, int n, int multimass,
@@ -602,17 +599,21 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   }
   if (n > 0x7fffffffull) return Status::err(-1, "too many particles for one tree (max 2^31-1)");
 
+  // up to 2^19 particles the scratch is one allocation (about 200 B a particle)
+  Arena arena(st);
+  if (n <= ((size_t)1 << 19)) CK(arena.mem.alloc(((size_t)1 << 20) + 240 * n + 2 * sizeof(Slot) * (n / (size_t)prm.bucket)));
+
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   CK(cudaEventRecord(e0, st));
 
-  ABuf<glb_particle_rec> dp(st);
+  ABuf<glb_particle_rec> dp(st, &arena);
   CK(dp.alloc(n));
   CK(cudaMemcpyAsync(dp.p, hp, n * sizeof(glb_particle_rec), cudaMemcpyHostToDevice, st));
 
   // ---- root box (BuildQTreeNB, quadTree.h:297-337)
-  ABuf<unsigned> mm(st);
+  ABuf<unsigned> mm(st, &arena);
   CK(mm.alloc(4));
   unsigned init[4] = {0xffffffffu, 0xffffffffu, 0u, 0u};
   CK(cudaMemcpyAsync(mm.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
@@ -632,8 +633,8 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   p2[jj] = p1[jj] + lengths[!jj];
 
   // ---- keys + stable sort
-  ABuf<unsigned long long> keys(st), keys2(st);
-  ABuf<unsigned> idx(st), sidx(st);
+  ABuf<unsigned long long> keys(st, &arena), keys2(st, &arena);
+  ABuf<unsigned> idx(st, &arena), sidx(st, &arena);
   CK(keys.alloc(n));
   CK(keys2.alloc(n));
   CK(idx.alloc(n));
@@ -641,7 +642,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   k_keys<<<nblk(n, 256), 256, 0, st>>>(dp.p, n, p1[0], p1[1], p2[0], p2[1], keys.p, idx.p);
   size_t tmp_bytes = 0;
   CK(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.p, keys2.p, idx.p, sidx.p, (int)n, 0, 64, st));
-  ABuf<char> tmp(st);
+  ABuf<char> tmp(st, &arena);
   CK(tmp.alloc(tmp_bytes));
   CK(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, keys.p, keys2.p, idx.p, sidx.p, (int)n, 0, 64, st));
   keys.release();
@@ -651,7 +652,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   std::vector<int> off = {0, 1};
   // grown below where a tree needs more
   size_t cap = std::min<size_t>((size_t)1 << 20, std::max<size_t>(1024, 2 * (n / (size_t)prm.bucket)));
-  ABuf<Slot> slots(st);
+  ABuf<Slot> slots(st, &arena);
   CK(slots.alloc(cap));
   Slot root;
   memset(&root, 0, sizeof(root));
@@ -663,7 +664,7 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   root.pre = 0;
   root.pref = 0;
   CK(cudaMemcpyAsync(slots.p, &root, sizeof(Slot), cudaMemcpyHostToDevice, st));
-  ABuf<int> counters(st);
+  ABuf<int> counters(st, &arena);
   CK(counters.alloc(2));
   for (int L = 0;; ++L) {
     int lo = off[L], hi = off[L + 1];
@@ -679,11 +680,12 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
     if (need > 0x7fffffffull) return Status::err(-1, "tree too large");
     if (need > cap) {
       size_t ncap = std::max(need, cap * 2);
-      ABuf<Slot> ns(st);
+      ABuf<Slot> ns(st, &arena);
       CK(ns.alloc(ncap));
       CK(cudaMemcpyAsync(ns.p, slots.p, (size_t)hi * sizeof(Slot), cudaMemcpyDeviceToDevice, st));
       std::swap(ns.p, slots.p);
       std::swap(ns.n, slots.n);
+      std::swap(ns.carved, slots.carved);
       cap = ncap;
     }
     k_split<<<nblk(hi - lo, 256), 256, 0, st>>>(slots.p, lo, hi, keys2.p);
@@ -717,13 +719,13 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   k_gather_parts<<<nblk(n, 256), 256, 0, st>>>(dp.p, sidx.p, (int)n, multimass, multiradius, parts);
 
   // ---- big-particle lists of internal boxes
-  ABuf<int> pre2slot(st);
+  ABuf<int> pre2slot(st, &arena);
   CK(pre2slot.alloc(nnodes));
   k_pre2slot<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, pre2slot.p);
   int nbig = 0;
   if (multiradius) {
-    ABuf<unsigned> fkey(st), fval(st), ckey(st), cval(st), skey(st), sval(st);
-    ABuf<int> flags(st), nsel(st);
+    ABuf<unsigned> fkey(st, &arena), fval(st, &arena), ckey(st, &arena), cval(st, &arena), skey(st, &arena), sval(st, &arena);
+    ABuf<int> flags(st, &arena), nsel(st, &arena);
     CK(fkey.alloc(n));
     CK(fval.alloc(n));
     CK(flags.alloc(n));
@@ -773,15 +775,14 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   ExpTab *exptab = (ExpTab *)(nm + o_e);
   k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes,
                                                   cnodes, fsnodes);
-  k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(tnodes, ncut, cutanc);
-  k_exp_tables<<<4, 256, 0, st>>>(exptab);
-  ABuf<int> dbad(st);
+  k_cut_ancestors<<<nblk(std::max(ncut, 1024), 128), 128, 0, st>>>(tnodes, ncut, cutanc, exptab);
+  ABuf<int> dbad(st, &arena);
   CK(dbad.alloc(1));
   CK(cudaMemsetAsync(dbad.p, 0, sizeof(int), st));
   if (nnodes > 0) k_check_skips<<<nblk(nnodes, 256), 256, 0, st>>>(snodes, nnodes, dbad.p);
   int hbad = 0;
   CK(cudaMemcpyAsync(&hbad, dbad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  ABuf<double> phin(st);
+  ABuf<double> phin(st, &arena);
   CK(phin.alloc(8));
   k_phi_node<<<1, 1, 0, st>>>(slots.p, phin.p);
   double hphi[8];
