@@ -88,8 +88,9 @@ struct __align__(16) FNodeS {
 constexpr int kCutStep = 16;
 
 // Tables of the strip walk's exponential: exp(-j/1024) and exp(-m).
+constexpr int kExpHi = 704;
 struct ExpTab {
-  double lo[1024], hi[704];
+  double lo[1024], hi[kExpHi];
 };
 
 struct TreeDev {

@@ -473,7 +473,7 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
 __global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc, ExpTab *E) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g < 1024) E->lo[g] = exp(-(double)g / 1024.0);
-  if (g < 704) E->hi[g] = exp(-(double)g);
+  if (g < kExpHi) E->hi[g] = exp(-(double)g);
   if (g >= ncut) return;
   const int s = g * kCutStep;
   int *a = anc + (size_t)kMaxDepth * g, k = 0, node = 0;

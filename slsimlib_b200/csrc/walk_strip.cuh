@@ -63,7 +63,9 @@ __device__ __forceinline__ double strip_rcp(double a) {
 // The constants of the two highest terms have a zero low word (r^3/6 is below
 // 2e-11 and the rounding of its constant 6e-7 of it), so that they are
 // immediates; full double constants cost two instructions each per use.  t is
-// held at 700 (by its high word), where exp(-t) is below 1e-304.
+// held at 700 (by its high word), where exp(-t) is below 1e-304.  A NaN with
+// its sign set passes that as a negative number, and k is then any word of its
+// payload: the table index has a bound of its own (the result stays NaN, by r).
 constexpr double kC3 = -0x1.55555p-3, kC4 = 0x1.55555p-5;
 __device__ __forceinline__ double strip_exp_neg(double t, const ExpTab &E) {
   constexpr double kShift = 6755399441055744.0;  // 1.5 * 2^52
@@ -74,7 +76,7 @@ __device__ __forceinline__ double strip_exp_neg(double t, const ExpTab &E) {
   double p = __fma_rn(r, kC4, kC3);
   p = __fma_rn(p, r, 0.5);
   p = __fma_rn(p, r, -1.0);
-  const double e = __dmul_rn(E.hi[k >> 10], E.lo[k & 1023]);
+  const double e = __dmul_rn(E.hi[min((unsigned)k >> 10, (unsigned)kExpHi - 1u)], E.lo[k & 1023]);
   return __fma_rn(e, __dmul_rn(r, p), e);
 }
 

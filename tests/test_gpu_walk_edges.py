@@ -1,0 +1,74 @@
+"""Inputs, limits and call forms at which the FP64 walks, their scratch and the
+dispatch between them can go wrong."""
+import numpy as np
+import pytest
+
+import slsimlib_b200 as glb
+from slsimlib_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _cluster(seed, n, size=0.01):
+    r = np.random.default_rng(seed)
+    p = np.zeros(n, dtype=synth.PARTICLE_DTYPE)
+    p["x"] = np.concatenate([r.normal(0, 0.1, (n - n // 3, 3)), r.uniform(-1, 1, (n // 3, 3))])[:n]
+    p["Mass"] = r.uniform(0.5, 2.0, n)
+    p["Size"] = size * 10 ** r.uniform(-1, 1, n)
+    return p
+
+
+def _device_force(t, x, precision=glb.PREC_FP64, stream=None):
+    import torch
+    d = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    o = torch.full((len(x), 5), np.nan, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    t.force_device(len(x), d.data_ptr(), o.data_ptr(), precision, stream)
+    torch.cuda.synchronize()
+    return o.cpu().numpy()
+
+
+def _recur(t, x):
+    a, k, g, ph = t.force2D_recur(x)
+    return np.concatenate([a, k[:, None], g[:, :2], ph[:, None]], axis=1)
+
+
+# NaNs of either sign whose low words, read as table indices, lie far outside any table.
+NAN_BITS = np.array([0xFFFFFFFFE0000000, 0xFFF8000000000000, 0xFFFFFFFFFFFFFFFF, 0xFFF800007FFFFFFF, 0x7FF8000080000000,
+                     0xFFF0000000100000], dtype=np.uint64)
+
+
+@pytest.mark.parametrize("n", [64, 1 << 16])
+@pytest.mark.parametrize("kw", [dict(inv_screening_scale=1.0), dict(inv_screening_scale=2.0, inv_area=0.1)])
+def test_nan_payloads_stay_inside_the_tables(n, kw):
+    t = glb.TreeQuadParticles(_cluster(1, 5000), bucket=5, theta_force=0.1, **kw)
+    x = np.random.default_rng(2).normal(0, 0.3, (n, 2))
+    y = x.copy()
+    bad = np.arange(3, n, 41)
+    y[bad, 0] = np.resize(NAN_BITS, len(bad)).view(np.float64)
+    y[bad[::2], 1] = y[bad[::2], 0]
+    ok = np.setdiff1d(np.arange(n), bad)
+    for f in (_device_force, _recur):
+        a, b = f(t, x), f(t, y)
+        assert np.array_equal(a[ok], b[ok])
+        assert np.all(np.isnan(b[bad][:, [0, 1, 3, 4]]))
+
+
+def test_nan_payloads_in_lenses_and_served_requests():
+    spec = synth.light_cone(seed=5, n_total=30000, n_planes=2, halos_per_plane=4)
+    lens = glb.lens_from_spec(spec)
+    for n in (97, 1 << 16, 131072):  # shared walks, one and two rays per lane
+        x = np.random.default_rng(3).normal(0, 10 * synth.ARCSEC, (n, 2))
+        y = x.copy()
+        bad = np.arange(5, n, 29)
+        y[bad, 1] = np.resize(NAN_BITS, len(bad)).view(np.float64)
+        ok = np.setdiff1d(np.arange(n), bad)
+        (y0, A0), (y1, A1) = lens.rayshooterInternal(x), lens.rayshooterInternal(y)
+        assert np.array_equal(y0[ok], y1[ok]) and np.array_equal(A0[ok], A1[ok])
+        assert np.all(np.isnan(A1[bad]).any(axis=1))
+        if n == 97:
+            srv = glb.Server([lens], precision=glb.PREC_FP64)
+            got = [srv.wait(srv.submit(0, r))[:2] for r in (x, y)]
+            srv.close()
+            assert np.array_equal(got[0][0][ok], got[1][0][ok]) and np.array_equal(got[0][1][ok], got[1][1][ok])
+            assert np.all(np.isnan(got[1][1][bad]).any(axis=1))
