@@ -73,9 +73,11 @@ enum {
 const char *glb_last_error(void);
 /* Library version string. */
 const char *glb_version(void);
-/* Options: GLB_OPT_KEEP_TREE_EXPORT (1) keeps per-branch build data so that
- * glb_tree_export can be called (test and debugging use). */
-enum { GLB_OPT_KEEP_TREE_EXPORT = 1 };
+/* Options (test and debugging use): GLB_OPT_KEEP_TREE_EXPORT (1) keeps per-branch
+ * build data so that glb_tree_export can be called; GLB_OPT_ALLOC_LIMIT (2)
+ * refuses the calling thread's device allocations of more than `value` bytes,
+ * as a GPU without that much free memory would (0: no limit). */
+enum { GLB_OPT_KEEP_TREE_EXPORT = 1, GLB_OPT_ALLOC_LIMIT = 2 };
 int glb_set_option(int option, long long value);
 
 /* ---------------------------------------------------------------- trees */

@@ -32,7 +32,13 @@ struct Status {
   bool good() const { return code == 0; }
 };
 
-// Device memory owned by RAII.
+// The largest device allocation this thread may make, 0 for no limit
+// (GLB_OPT_ALLOC_LIMIT: for tests of refused allocations).
+inline thread_local size_t alloc_limit = 0;
+inline bool alloc_refused(size_t bytes) { return alloc_limit && bytes > alloc_limit; }
+
+// Device memory owned by RAII.  After a refused allocation the buffer is empty
+// and the runtime's last error is cleared (the caller has the status).
 template <typename T>
 struct DBuf {
   T *p = nullptr;
@@ -48,9 +54,16 @@ struct DBuf {
   }
   cudaError_t alloc(size_t count) {
     release();
-    n = count;
     if (count == 0) return cudaSuccess;
-    return cudaMalloc((void **)&p, count * sizeof(T));
+    cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation
+                                                     : cudaMalloc((void **)&p, count * sizeof(T));
+    if (e == cudaSuccess) {
+      n = count;
+    } else {
+      p = nullptr;
+      (void)cudaGetLastError();
+    }
+    return e;
   }
 };
 
@@ -106,9 +119,14 @@ cudaError_t ABuf<T>::alloc(size_t count) {
       return cudaSuccess;
     }
   cudaMemPool_t pool;
-  cudaError_t e = scratch_pool(&pool);
+  cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation : scratch_pool(&pool);
   if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);
-  if (e == cudaSuccess) n = count;
+  if (e == cudaSuccess) {
+    n = count;
+  } else {
+    p = nullptr;
+    (void)cudaGetLastError();
+  }
   return e;
 }
 

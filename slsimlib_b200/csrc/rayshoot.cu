@@ -1420,6 +1420,7 @@ int ensure_ws(LensWS *w, size_t n, bool per_ray) {
   if (n > 0xffffffffull) return fail(GLB_ERR_ARG, "too many rays in one call (max 2^32-1)");
   if (w->ws_n < n || (per_ray && w->jmax_ray.n < n)) {
     size_t m = std::max(n, w->ws_n);
+    w->ws_n = 0;  // until every buffer below holds m rays
     CKR(w->st.alloc(12 * m));
     CKR(w->keys.alloc(m));
     CKR(w->keys2.alloc(m));
@@ -1735,6 +1736,11 @@ const char *glb_version(void) { return "glamer_b200 0.1 (sm_100a)"; }
 int glb_set_option(int option, long long value) {
   if (option == GLB_OPT_KEEP_TREE_EXPORT) {
     g_keep_tree_export = value ? 1 : 0;
+    return 0;
+  }
+  if (option == GLB_OPT_ALLOC_LIMIT) {
+    if (value < 0) return fail(GLB_ERR_ARG, "negative limit");
+    alloc_limit = (size_t)value;
     return 0;
   }
   return fail(GLB_ERR_ARG, "unknown option");

@@ -734,6 +734,7 @@ Status smooth_particles_device(const glb_particle_rec *d_p, size_t n, int nsmoot
   Workspace &w = wss[dev];
   std::lock_guard<std::mutex> lock(w.mu);
   if (w.n < n) {
+    w.n = 0;  // until every buffer below holds n particles
     CK(w.key.alloc(n));
     CK(w.key2.alloc(n));
     CK(w.idx.alloc(n));
@@ -743,11 +744,13 @@ Status smooth_particles_device(const glb_particle_rec *d_p, size_t n, int nsmoot
   }
   const size_t nch = (n + 31) / 32;
   if (w.nch < nch) {
+    w.nch = 0;
     CK(w.clo.alloc(nch));
     CK(w.chi.alloc(nch));
     w.nch = nch;
   }
   if (w.P < P) {
+    w.P = 0;
     CK(w.blo.alloc(2 * (size_t)P));
     CK(w.bhi.alloc(2 * (size_t)P));
     w.P = P;

@@ -28,6 +28,25 @@ def _device_force(t, x, precision=glb.PREC_FP64, stream=None):
     return o.cpu().numpy()
 
 
+class alloc_limit:
+    """Device allocations of this thread above `nbytes` are refused inside the block."""
+
+    def __init__(self, nbytes):
+        self.nbytes = nbytes
+
+    def __enter__(self):
+        assert glb.load_library().glb_set_option(2, self.nbytes) == 0
+
+    def __exit__(self, *a):
+        glb.load_library().glb_set_option(2, 0)
+
+
+def _refused(f):
+    with pytest.raises(glb.GlamerError) as e:
+        f()
+    assert "out of memory" in str(e.value)
+
+
 def _recur(t, x):
     a, k, g, ph = t.force2D_recur(x)
     return np.concatenate([a, k[:, None], g[:, :2], ph[:, None]], axis=1)
@@ -72,3 +91,44 @@ def test_nan_payloads_in_lenses_and_served_requests():
             srv.close()
             assert np.array_equal(got[0][0][ok], got[1][0][ok]) and np.array_equal(got[0][1][ok], got[1][1][ok])
             assert np.all(np.isnan(got[1][1][bad]).any(axis=1))
+
+
+def _lens(n=20000, planes=2):
+    return glb.lens_from_spec(synth.light_cone(seed=6, n_total=n, n_planes=planes, halos_per_plane=4))
+
+
+@pytest.mark.parametrize("limit", [1 << 20, 80 * 60000])  # the call's staging, the workspace behind it
+@pytest.mark.parametrize("precision", [glb.PREC_FP64, glb.PREC_SPLIT])
+def test_lens_calls_after_a_refused_allocation(limit, precision):
+    lens = _lens()
+    x = np.random.default_rng(1).normal(0, 10 * synth.ARCSEC, (60000, 2))
+    zs = np.full(len(x), 2.0)
+    want = lens.rayshooterInternal(x[:3000], None, precision)
+    grid = glb.GridMap(lens, 48, (0.0, 0.0), 20 * synth.ARCSEC, precision).y
+    for again in range(2):
+        with alloc_limit(limit):
+            _refused(lambda: lens.rayshooterInternal(x, None, precision))
+            _refused(lambda: lens.rayshooterInternal(x, zs, precision))
+            _refused(lambda: glb.GridMap(lens, 300, (0.0, 0.0), 20 * synth.ARCSEC, precision))
+        for got, ref in zip(lens.rayshooterInternal(x[:3000], None, precision), want):
+            assert np.array_equal(got, ref)
+        assert np.array_equal(glb.GridMap(lens, 48, (0.0, 0.0), 20 * synth.ARCSEC, precision).y, grid)
+
+
+def test_trees_and_smoothing_after_a_refused_allocation():
+    p = _cluster(2, 40000)
+    x = np.random.default_rng(4).normal(0, 0.3, (50000, 2))
+    t = glb.TreeQuadParticles(p, bucket=5, theta_force=0.3)
+    want = _recur(t, x[:2000])
+    small, size = p[:3000].copy(), p.copy()
+    glb.calculate_smoothing(16, small)
+    with alloc_limit(1 << 19):
+        _refused(lambda: glb.TreeQuadParticles(p, bucket=5, theta_force=0.3))
+        _refused(lambda: _recur(t, x))
+        _refused(lambda: glb.calculate_smoothing(16, size))
+    again = p[:3000].copy()
+    glb.calculate_smoothing(16, again)
+    assert np.array_equal(small["Size"], again["Size"])
+    assert np.array_equal(_recur(t, x[:2000]), want)
+    u = glb.TreeQuadParticles(p, bucket=5, theta_force=0.3)
+    assert np.array_equal(_recur(u, x[:2000]), want)
