@@ -1635,11 +1635,12 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
   }
   if (int rc = upload_lens(l)) return rc;
   if (int rc = ensure_ws(w, n, zs != nullptr)) return rc;
-  // shared walks: calls below kPlanePartsMax rays, which run in one slab
-  const size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
+  // shared walks: calls below kPlanePartsMax rays, which run in one slab;
+  // without memory for their scratch the walks are not shared
+  size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
   if (psums) {
     const size_t pb = psums + parts_bytes(n, 0, 0) + psums / (5 * sizeof(double)) + 256;  // sums, counters, flags
-    if (w->parts.n < pb) CKR(w->parts.alloc(pb));
+    if (w->parts.n < pb && w->parts.alloc(pb) != cudaSuccess) psums = 0;
   }
   CKR(cudaStreamWaitEvent(s, w->done, 0));
   CKR(cudaEventRecord(w->ev[0], s));
@@ -1816,7 +1817,10 @@ static int force_particles(const TreeDev &T, cudaStream_t s, DBuf<char> &ws, siz
   const size_t o_perm = o_k + al(8 * n), o_bb = o_perm + al(8 * n), o_tmp = o_bb + 256, o_part = o_tmp + al(tb);
   const size_t sums = (size_t)p.nparts * 6 * n * sizeof(double);
   const size_t need = o_part + (p.nparts > 1 ? parts_bytes(n, p.nparts, 6) : 0);
-  if (ws.n < need) CKR(ws.alloc(need));
+  if (ws.n < need && ws.alloc(need) != cudaSuccess) {
+    p.nparts = 1;  // no memory for shared walks
+    CKR(ws.alloc(o_part));
+  }
   char *m = ws.p;
   double *dx = (double *)(m + o_x), *px = (double *)(m + o_xy), *py = px + n, *out = (double *)(m + o_out);
   unsigned *keys = (unsigned *)(m + o_k), *perm0 = (unsigned *)(m + o_perm), *perm = perm0 + n;
@@ -1867,12 +1871,19 @@ static int force_generic(const HaloDev &H, int device, cudaStream_t s, size_t n,
   if (int rc = set_dev(device)) return rc;
   if (H.kind == HALO_PARTICLES) {
     DBuf<char> local;
-    constexpr size_t kChunk = (size_t)1 << 24;  // bounds the workspace
-    for (size_t o = 0; o < n; o += kChunk)
-      if (int rc = force_particles(H.tree, s, ws ? *ws : local, std::min(kChunk, n - o), xcm + 2 * o,
-                                   alpha ? alpha + 2 * o : nullptr, kappa ? kappa + o : nullptr,
-                                   gamma ? gamma + 3 * o : nullptr, phi ? phi + o : nullptr))
-        return rc;
+    size_t chunk = (size_t)1 << 24;  // bounds the workspace, smaller where its memory is refused
+    for (size_t o = 0; o < n;) {
+      const size_t m = std::min(chunk, n - o);
+      const int rc = force_particles(H.tree, s, ws ? *ws : local, m, xcm + 2 * o, alpha ? alpha + 2 * o : nullptr,
+                                     kappa ? kappa + o : nullptr, gamma ? gamma + 3 * o : nullptr,
+                                     phi ? phi + o : nullptr);
+      if (rc == GLB_ERR_OOM && m > 65536) {
+        chunk = m / 2;
+        continue;
+      }
+      if (rc) return rc;
+      o += m;
+    }
     return 0;
   }
   NFWTables tab{};
@@ -1945,10 +1956,12 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
     // a stream in capture cannot wait for earlier calls' use of the scratch
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (p.nparts > 1) CKR(cudaStreamIsCapturing(s, &cap));
-    if (p.nparts > 1 && cap == cudaStreamCaptureStatusNone) {
-      std::lock_guard<std::mutex> lk(t->dev_mu);
-      const size_t need = parts_bytes(n, p.nparts, 5);
-      if (t->dev_ws.n < need) CKR(t->dev_ws.alloc(need));
+    const bool shared = p.nparts > 1 && cap == cudaStreamCaptureStatusNone;
+    std::unique_lock<std::mutex> lk(t->dev_mu, std::defer_lock);
+    if (shared) lk.lock();
+    const size_t need = parts_bytes(n, p.nparts, 5);
+    // without memory for the scratch the walks are not shared
+    if (shared && (t->dev_ws.n >= need || t->dev_ws.alloc(need) == cudaSuccess)) {
       if (!t->dev_done) CKR(cudaEventCreateWithFlags(&t->dev_done, cudaEventDisableTiming));
       CKR(cudaStreamWaitEvent(s, t->dev_done, 0));
       p.px = rays_dev;

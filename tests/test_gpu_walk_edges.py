@@ -132,3 +132,47 @@ def test_trees_and_smoothing_after_a_refused_allocation():
     assert np.array_equal(_recur(t, x[:2000]), want)
     u = glb.TreeQuadParticles(p, bucket=5, theta_force=0.3)
     assert np.array_equal(_recur(u, x[:2000]), want)
+
+
+def _noalloc(lens, x):
+    import torch
+    d = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    y = torch.empty((len(x), 2), dtype=torch.float64, device="cuda")
+    A = torch.empty((len(x), 4), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    glb._check(glb.load_library().glb_lens_rayshoot_noalloc(lens._h, len(x), d.data_ptr(), None, y.data_ptr(),
+                                                            A.data_ptr(), glb.PREC_FP64, None))
+    torch.cuda.synchronize()
+    return y.cpu().numpy(), A.cpu().numpy()
+
+
+@pytest.mark.parametrize("n", [1, 700, 4097])
+def test_walks_are_not_shared_without_memory_for_it(n):
+    """The sums of shared walks take up to 100 MB; a call that cannot have them
+    gives the results of one warp per 32 rays, which needs none."""
+    limit = {1: 1 << 14}.get(n, 1 << 20)
+    lens, p = _lens(200000), _cluster(4, 60000)
+    x = np.random.default_rng(5).normal(0, 10 * synth.ARCSEC, (n, 2))
+    want = _noalloc(lens, x)
+    t, u = (glb.TreeQuadParticles(p, bucket=5, theta_force=0.1) for _ in range(2))
+    r = np.random.default_rng(6).normal(0, 0.3, (1 << 16, 2))
+    whole, few, host = _device_force(t, r)[:n], _device_force(t, r[:n]), _recur(t, r[:n])
+    assert n == 1 or not np.array_equal(few, whole)  # shared: another order of the sum
+    with alloc_limit(limit):
+        for again in range(2):
+            got = lens.rayshooterInternal(x)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+            assert np.array_equal(_device_force(u, r[:n]), whole)
+            assert np.abs(_recur(u, r[:n]) - host).max() <= 1e-11 * np.abs(host).max()
+    shared = lens.rayshooterInternal(x)
+    assert n == 1 or not np.array_equal(shared[1], want[1])
+
+
+def test_host_forces_in_smaller_pieces_where_memory_is_refused():
+    t = glb.TreeQuadParticles(_cluster(7, 3000), bucket=20, theta_force=0.3)
+    x = np.random.default_rng(8).normal(0, 0.3, (300001, 2))
+    want = _recur(t, x)
+    u = glb.TreeQuadParticles(_cluster(7, 3000), bucket=20, theta_force=0.3)
+    with alloc_limit(110 * 100000):
+        got = _recur(u, x)
+    assert np.abs(got - want).max() <= 1e-11 * np.abs(want).max()
