@@ -67,10 +67,10 @@ struct DBuf {
   }
 };
 
-// The pool of this device's build scratch.  It keeps up to 256 MB between
-// uses, so that building many trees does not map memory for each (a build
-// takes some twenty buffers); what it holds beyond that goes back to the device
-// at the next synchronisation.
+// The pool of this device's scratch memory (tree builds, shared walks).  It
+// keeps up to 256 MB between uses, so that building many trees does not map
+// memory for each (a build takes some twenty buffers); what it holds beyond that
+// goes back to the device at the next synchronisation.
 cudaError_t scratch_pool(cudaMemPool_t *pool);
 
 // Scratch memory from the pool, taken and given back in the order of a stream.

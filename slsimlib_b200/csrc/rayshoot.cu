@@ -185,7 +185,6 @@ struct LensWS {
   DBuf<char> sort_tmp;
   DBuf<unsigned long long> bbox;
   DBuf<unsigned char> status;  // per-ray status staging
-  DBuf<char> parts;         // scratch of shared walks
   size_t ws_n = 0;
   float last_kernel_ms = 0, last_total_ms = 0;
   bool timed = false;
@@ -1487,7 +1486,9 @@ const glb_halo *single_tree(const glb_lens *l, int j) {
   return ph && ph->tree && !l->plane_field[j] && !ph->tree->dev.periodic ? ph : nullptr;
 }
 
-// The scratch of shared walks: [sums of the parts][counters][used flags].
+// The scratch of shared walks: [sums of the parts][counters][used flags], from
+// the device's scratch pool in the order of the call's stream, so that calls on
+// several streams neither wait for one another nor stall the device.
 constexpr int kPartCounters = 256;  // launches between two clearings of the counters
 size_t parts_bytes(size_t n, int parts, int comps) {
   return (size_t)parts * comps * n * sizeof(double) + kPartCounters * sizeof(int) + (size_t)parts * ((n + 31) / 32);
@@ -1638,9 +1639,10 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
   // shared walks: calls below kPlanePartsMax rays, which run in one slab;
   // without memory for their scratch the walks are not shared
   size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
+  ABuf<char> parts(s);
   if (psums) {
     const size_t pb = psums + parts_bytes(n, 0, 0) + psums / (5 * sizeof(double)) + 256;  // sums, counters, flags
-    if (w->parts.n < pb && w->parts.alloc(pb) != cudaSuccess) psums = 0;
+    if (parts.alloc(pb) != cudaSuccess) psums = 0;
   }
   CKR(cudaStreamWaitEvent(s, w->done, 0));
   CKR(cudaEventRecord(w->ev[0], s));
@@ -1710,7 +1712,7 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
     ai.n = mi;
     ai.jmax_ray = zs ? w->jmax_ray.p + o : nullptr;
     ai.src_ray = zs ? w->src_ray.p + 2 * o : nullptr;
-    if (int rc = launch_plane_steps(l, ai, jmax_launch, precision, si, d_counts, psums ? w->parts.p : nullptr, psums))
+    if (int rc = launch_plane_steps(l, ai, jmax_launch, precision, si, d_counts, parts.p, psums))
       return rc;
     k_finish<<<nblk(mi, 256), 256, 0, si>>>(ai.st, w->perm.p + o, mi, y, A, status, skip);
     if (i > 0) {
@@ -1754,11 +1756,6 @@ struct glb_tree {
   cudaStream_t stream = nullptr;
   std::mutex mu;     // guards ws
   DBuf<char> ws;     // force2D_recur's device workspace
-  // scratch of the device-array call's shared walks; calls that use it are
-  // ordered on the GPU by dev_done, whatever their streams
-  std::mutex dev_mu;
-  DBuf<char> dev_ws;
-  cudaEvent_t dev_done = nullptr;
 };
 
 int glb_tree_create(const glb_particle *particles, size_t n, float mass_fixed, float size_fixed, double inv_area,
@@ -1794,8 +1791,6 @@ int glb_tree_destroy(glb_tree *t) {
   cudaSetDevice(t->device);
   t->tree.reset();
   t->ws.release();
-  t->dev_ws.release();
-  if (t->dev_done) cudaEventDestroy(t->dev_done);
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;
   return 0;
@@ -1953,17 +1948,12 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
   if (precision == GLB_PREC_FP64 && !t->tree->dev.periodic) {
     PartArgs p;
     p.nparts = strip_parts(n, kPlanePartsMax, t->tree->dev.nnodes, &p.len);
-    // a stream in capture cannot wait for earlier calls' use of the scratch
+    // (in a capture the scratch would become the graph's: one launch, unshared)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (p.nparts > 1) CKR(cudaStreamIsCapturing(s, &cap));
-    const bool shared = p.nparts > 1 && cap == cudaStreamCaptureStatusNone;
-    std::unique_lock<std::mutex> lk(t->dev_mu, std::defer_lock);
-    if (shared) lk.lock();
-    const size_t need = parts_bytes(n, p.nparts, 5);
     // without memory for the scratch the walks are not shared
-    if (shared && (t->dev_ws.n >= need || t->dev_ws.alloc(need) == cudaSuccess)) {
-      if (!t->dev_done) CKR(cudaEventCreateWithFlags(&t->dev_done, cudaEventDisableTiming));
-      CKR(cudaStreamWaitEvent(s, t->dev_done, 0));
+    ABuf<char> ws(s);
+    if (p.nparts > 1 && cap == cudaStreamCaptureStatusNone && ws.alloc(parts_bytes(n, p.nparts, 5)) == cudaSuccess) {
       p.px = rays_dev;
       p.py = rays_dev + 1;
       p.stride = 2;
@@ -1973,11 +1963,10 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
       p.j = 0;
       p.jmax = 1;
       p.n = n;
-      set_part_scratch(p, t->dev_ws.p, (size_t)p.nparts * 5 * n * sizeof(double), 0);
+      set_part_scratch(p, ws.p, (size_t)p.nparts * 5 * n * sizeof(double), 0);
       CKR(cudaMemsetAsync(p.counter, 0, sizeof(int), s));
       if (int rc = launch_parts<false>(t->tree->dev, p, s)) return rc;
       k_force5_parts_end<<<nblk(n, 32), dim3(32, kSumRows), 0, s>>>(t->tree->dev, n, p.out, p.used, p.nparts, out_dev);
-      CKR(cudaEventRecord(t->dev_done, s));
       CKR(cudaGetLastError());
       return 0;
     }

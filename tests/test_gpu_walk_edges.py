@@ -176,3 +176,81 @@ def test_host_forces_in_smaller_pieces_where_memory_is_refused():
     with alloc_limit(110 * 100000):
         got = _recur(u, x)
     assert np.abs(got - want).max() <= 1e-11 * np.abs(want).max()
+
+
+def test_device_forces_on_two_streams_overlap():
+    """Small FP64 device calls on two streams use scratch of their own: a call
+    on the second stream ends while the first still has work queued."""
+    import torch
+    t = glb.TreeQuadParticles(_cluster(9, 200000), bucket=5, theta_force=0.05)
+    x = np.random.default_rng(10).normal(0, 0.3, (20000, 2))
+    want, few = _device_force(t, x), _device_force(t, x[:64])
+    d = torch.from_numpy(x).cuda()
+    out = torch.zeros((40, len(x), 5), dtype=torch.float64, device="cuda")
+    small = torch.zeros((64, 5), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for o in out:
+        t.force_device(len(x), d.data_ptr(), o.data_ptr(), glb.PREC_FP64, a.cuda_stream)
+    t.force_device(64, d.data_ptr(), small.data_ptr(), glb.PREC_FP64, b.cuda_stream)
+    b.synchronize()
+    assert not a.query()
+    assert np.array_equal(small.cpu().numpy(), few)
+    a.synchronize()
+    assert all(np.array_equal(o, want) for o in out.cpu().numpy())
+
+
+def test_device_forces_of_several_threads_and_sizes():
+    import threading
+    import torch
+    t = glb.TreeQuadParticles(_cluster(11, 50000), bucket=5, theta_force=0.1)
+    x = np.random.default_rng(12).normal(0, 0.3, (5000, 2))
+    sizes = (17, 5000, 500, 4999, 33, 2500)
+    want = {n: _device_force(t, x[:n]) for n in sizes}
+    d = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        torch.cuda.set_device(0)
+        s = torch.cuda.Stream()
+        for n in sizes[k:] + sizes[:k]:
+            o = torch.zeros((n, 5), dtype=torch.float64, device="cuda")
+            torch.cuda.current_stream().synchronize()
+            t.force_device(n, d.data_ptr(), o.data_ptr(), glb.PREC_FP64, s.cuda_stream)
+            s.synchronize()
+            if not np.array_equal(o.cpu().numpy(), want[n]):
+                wrong.append(n)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for q in th:
+        q.start()
+    for q in th:
+        q.join()
+    assert not wrong
+
+
+def test_a_captured_device_force_is_one_unshared_launch():
+    import torch
+    t = glb.TreeQuadParticles(_cluster(13, 20000), bucket=5, theta_force=0.1)
+    x = np.random.default_rng(14).normal(0, 0.3, (1 << 16, 2))
+    want = _device_force(t, x)[:300]
+    d = torch.from_numpy(x[:300].copy()).cuda()
+    o = torch.zeros((300, 5), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s):
+        t.force_device(300, d.data_ptr(), o.data_ptr(), glb.PREC_FP64, s.cuda_stream)
+    for again in range(2):
+        o.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(o.cpu().numpy(), want)
+
+
+def test_growing_and_shrinking_lens_calls():
+    lens, other = _lens(), _lens()
+    x = np.random.default_rng(15).normal(0, 10 * synth.ARCSEC, (6000, 2))
+    for n in (500, 6000, 40, 3000, 5999, 1):
+        got, want = lens.rayshooterInternal(x[:n]), other.rayshooterInternal(x[:n])
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
