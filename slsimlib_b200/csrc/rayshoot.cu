@@ -1754,8 +1754,6 @@ struct glb_tree {
   std::unique_ptr<Tree> tree;
   int device = 0;
   cudaStream_t stream = nullptr;
-  std::mutex mu;     // guards ws
-  DBuf<char> ws;     // force2D_recur's device workspace
 };
 
 int glb_tree_create(const glb_particle *particles, size_t n, float mass_fixed, float size_fixed, double inv_area,
@@ -1790,7 +1788,6 @@ int glb_tree_destroy(glb_tree *t) {
   if (!t) return 0;
   cudaSetDevice(t->device);
   t->tree.reset();
-  t->ws.release();
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;
   return 0;
@@ -1798,10 +1795,13 @@ int glb_tree_destroy(glb_tree *t) {
 
 // A particle tree's forces and potential at host positions: rays sorted along
 // a Morton curve (neighbouring rays of a warp share the walk's decisions; each
-// ray's result is its own), walks shared by several warps in small calls.
-// ws: the caller's workspace, grown as needed.
-static int force_particles(const TreeDev &T, cudaStream_t s, DBuf<char> &ws, size_t n, const double *xcm,
-                           double *alpha, double *kappa, double *gamma, double *phi) {
+// ray's result is its own), walks shared by several warps in small calls.  The
+// workspace (104 bytes a ray, and up to 113 MB for shared walks) is the scratch
+// pool's: a buffer kept on the tree would have to be that large, and one
+// allocated for each call cost 2 to 5 ms of a 1.5 ms call (3,000 rays, opening
+// angle 0.3).
+static int force_particles(const TreeDev &T, cudaStream_t s, size_t n, const double *xcm, double *alpha, double *kappa,
+                           double *gamma, double *phi) {
   PartArgs p;
   p.nparts = T.periodic ? 1 : strip_parts(n, kForcePartsMax, T.nnodes, &p.len);
   size_t tb = 0;
@@ -1812,7 +1812,8 @@ static int force_particles(const TreeDev &T, cudaStream_t s, DBuf<char> &ws, siz
   const size_t o_perm = o_k + al(8 * n), o_bb = o_perm + al(8 * n), o_tmp = o_bb + 256, o_part = o_tmp + al(tb);
   const size_t sums = (size_t)p.nparts * 6 * n * sizeof(double);
   const size_t need = o_part + (p.nparts > 1 ? parts_bytes(n, p.nparts, 6) : 0);
-  if (ws.n < need && ws.alloc(need) != cudaSuccess) {
+  ABuf<char> ws(s);
+  if (ws.alloc(need) != cudaSuccess) {
     p.nparts = 1;  // no memory for shared walks
     CKR(ws.alloc(o_part));
   }
@@ -1859,19 +1860,17 @@ static int force_particles(const TreeDev &T, cudaStream_t s, DBuf<char> &ws, siz
 }
 
 static int force_generic(const HaloDev &H, int device, cudaStream_t s, size_t n, const double *xcm, double *alpha,
-                         double *kappa, double *gamma, double *phi, int subtract = 0, double screening = 1.0,
-                         DBuf<char> *ws = nullptr) {
+                         double *kappa, double *gamma, double *phi, int subtract = 0, double screening = 1.0) {
   if (n == 0) return 0;
   if (!xcm) return fail(GLB_ERR_ARG, "null positions");
   if (int rc = set_dev(device)) return rc;
   if (H.kind == HALO_PARTICLES) {
-    DBuf<char> local;
     size_t chunk = (size_t)1 << 24;  // bounds the workspace, smaller where its memory is refused
     for (size_t o = 0; o < n;) {
       const size_t m = std::min(chunk, n - o);
-      const int rc = force_particles(H.tree, s, ws ? *ws : local, m, xcm + 2 * o, alpha ? alpha + 2 * o : nullptr,
-                                     kappa ? kappa + o : nullptr, gamma ? gamma + 3 * o : nullptr,
-                                     phi ? phi + o : nullptr);
+      const int rc =
+          force_particles(H.tree, s, m, xcm + 2 * o, alpha ? alpha + 2 * o : nullptr, kappa ? kappa + o : nullptr,
+                          gamma ? gamma + 3 * o : nullptr, phi ? phi + o : nullptr);
       if (rc == GLB_ERR_OOM && m > 65536) {
         chunk = m / 2;
         continue;
@@ -1925,12 +1924,7 @@ int glb_tree_force2D_recur(glb_tree *t, size_t n, const double *rays, double *al
     }
     return 0;
   }
-  // one caller at a time uses the tree's workspace; others take their own
-  std::unique_lock<std::mutex> lk(t->mu, std::try_to_lock);
-  const int rc = force_generic(H, t->device, t->stream, n, rays, alpha, kappa, gamma, phi, 0, 1.0,
-                               lk.owns_lock() ? &t->ws : nullptr);
-  if (lk.owns_lock() && t->ws.n > ((size_t)64 << 20)) t->ws.release();  // a large call's is given back
-  return rc;
+  return force_generic(H, t->device, t->stream, n, rays, alpha, kappa, gamma, phi);
 }
 
 int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double *out_dev, int precision,

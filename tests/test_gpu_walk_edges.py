@@ -254,3 +254,37 @@ def test_growing_and_shrinking_lens_calls():
     for n in (500, 6000, 40, 3000, 5999, 1):
         got, want = lens.rayshooterInternal(x[:n]), other.rayshooterInternal(x[:n])
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_host_forces_of_two_callers_and_many_sizes():
+    import threading
+    t = glb.TreeQuadParticles(_cluster(16, 30000), bucket=5, theta_force=0.3)
+    x = np.random.default_rng(17).normal(0, 0.3, (20000, 2))
+    sizes = (1, 20000, 700, 4097, 64)
+    want = {n: _recur(t, x[:n]) for n in sizes}
+    wrong = []
+
+    def work(k):
+        for n in sizes[k:] + sizes[:k]:
+            if not np.array_equal(_recur(t, x[:n]), want[n]):
+                wrong.append(n)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for q in th:
+        q.start()
+    for q in th:
+        q.join()
+    assert not wrong
+
+
+def test_repeated_host_forces_keep_no_more_memory():
+    """The workspace of a host call (100 MB here) is not mapped and unmapped by
+    each: what the device has free does not change from call to call."""
+    import torch
+    t = glb.TreeQuadParticles(_cluster(18, 200000), bucket=5, theta_force=0.1)
+    x = np.random.default_rng(19).normal(0, 0.3, (5000, 2))
+    _recur(t, x)
+    free = torch.cuda.mem_get_info()[0]
+    for n in (3000, 5000, 400, 4999):
+        _recur(t, x[:n])
+        assert torch.cuda.mem_get_info()[0] == free
