@@ -37,7 +37,11 @@ struct Status {
 inline thread_local size_t alloc_limit = 0;
 inline bool alloc_refused(size_t bytes) { return alloc_limit && bytes > alloc_limit; }
 
-// Device memory owned by RAII.  After a refused allocation the buffer is empty
+// Gives back to the device what its scratch pool holds unused.
+void trim_scratch_pool();
+
+// Device memory owned by RAII.  An allocation that finds no memory is tried
+// again once the scratch pool has given back what it keeps.  After a refused allocation the buffer is empty
 // and the runtime's last error is cleared (the caller has the status).
 template <typename T>
 struct DBuf {
@@ -55,11 +59,20 @@ struct DBuf {
   cudaError_t alloc(size_t count) {
     release();
     if (count == 0) return cudaSuccess;
-    cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation
-                                                     : cudaMalloc((void **)&p, count * sizeof(T));
-    if (e == cudaSuccess) {
-      n = count;
-    } else {
+    cudaError_t e = try_alloc(count);
+    if (e == cudaErrorMemoryAllocation) {
+      trim_scratch_pool();
+      e = try_alloc(count);
+    }
+    if (e == cudaSuccess) n = count;
+    return e;
+  }
+
+ private:
+  cudaError_t try_alloc(size_t count) {
+    const cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation
+                                                           : cudaMalloc((void **)&p, count * sizeof(T));
+    if (e != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
     }

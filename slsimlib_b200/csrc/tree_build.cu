@@ -557,6 +557,12 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
+void trim_scratch_pool() {
+  cudaMemPool_t pool;
+  if (scratch_pool(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  (void)cudaGetLastError();
+}
+
 cudaError_t scratch_pool(cudaMemPool_t *pool) {
   static std::mutex mu;
   static cudaMemPool_t pools[64] = {};

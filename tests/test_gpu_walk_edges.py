@@ -288,3 +288,17 @@ def test_repeated_host_forces_keep_no_more_memory():
     for n in (3000, 5000, 400, 4999):
         _recur(t, x[:n])
         assert torch.cuda.mem_get_info()[0] == free
+
+
+def test_a_refused_allocation_takes_back_the_unused_scratch():
+    import torch
+    t = glb.TreeQuadParticles(_cluster(20, 200000), bucket=5, theta_force=0.1)
+    x = np.random.default_rng(21).normal(0, 0.3, (3000, 2))
+    want = _recur(t, x)
+    lens = _lens()
+    lens.rayshooterInternal(np.zeros((1, 2)))
+    free = torch.cuda.mem_get_info()[0]
+    with alloc_limit(1 << 20):
+        _refused(lambda: lens.rayshooterInternal(np.zeros((60000, 2))))
+    assert torch.cuda.mem_get_info()[0] >= free + (64 << 20)
+    assert np.array_equal(_recur(t, x), want)
