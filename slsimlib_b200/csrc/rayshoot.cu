@@ -1061,6 +1061,11 @@ __device__ __forceinline__ void tree_force(const TreeDev &T, size_t n, const dou
   for (int c = 0; c < 5; ++c) out[5 * k + c] = acc[c];
 }
 
+// FP64, node by node (walk_f64) and by strips (force_rule chooses).
+__global__ void __launch_bounds__(128) k_tree_force(const __grid_constant__ TreeDev T, size_t n, const double *x,
+                                                    double *out) {
+  tree_force<GLB_PREC_FP64>(T, n, x, out);
+}
 __global__ void __launch_bounds__(128, 5) k_tree_force_f64(const __grid_constant__ TreeDev T, size_t n,
                                                           const double *x, double *out) {
   __shared__ StripBlock<128> S;
@@ -1453,9 +1458,39 @@ int strip_parts(size_t n, size_t max_rays, int nnodes, int *len) {
 // Plane steps share walks below this many rays; from here on a call has a warp
 // for every slot of the GPU by itself.
 constexpr size_t kPlanePartsMax = (size_t)1 << 16;
-// Tree forces likewise (one walk per ray, so that a last, partly filled wave
-// weighs more than in a lens's planes).
+// Host tree forces likewise (one walk per ray, so that a last, partly filled
+// wave weighs more than in a lens's planes).
 constexpr size_t kForcePartsMax = (size_t)1 << 18;
+// FP64 forces at device positions: shared below `shared` rays; from there on, or
+// where they cannot be shared, by strips or node by node.  The rays come in the
+// caller's order, so a warp's may lie anywhere; then, and where leaves hold few
+// particles or the opening angle is wide (few cells a ray), most nodes of a strip
+// are mixed and it loses to the walk that takes them one at a time.  Gains over
+// that walk, shared (strips), 10^5 and 2.5e5 rays tiled over 1 to 100 arcsec or in
+// random order, by nodes (bucket 5 | bucket 20 of the triaxial cluster):
+//   angle 0.1  10.8k 1.1..2.4 (0.7..1.7) |  2.9k 1.4..2.6 (0.8..1.8)
+//               141k 0.9..1.4 (0.6..1.1) | 37.7k 1.3..2.1 (0.8..1.7)
+//               539k 0.9..1.2 (0.6..0.9) |  145k 1.1..1.6 (0.7..1.2)
+//              2.15M 0.8..1.1 (0.5..0.8) |  579k 1.0..1.4 (0.7..0.9)
+//         0.2  10.8k 1.0..1.5 (0.7..1.3) |  2.9k 1.3..2.0 (0.8..1.7)
+//               141k 0.8..1.1 (0.6..0.8) | 37.7k 1.0..1.4 (0.7..1.0)
+//               539k 0.8..1.0 (0.5..0.8) |  145k 0.8..1.2 (0.6..0.9)
+//         0.3  10.8k 0.9..1.1 (0.6..1.1) |  2.9k 1.3..1.6 (0.8..1.5)
+//               141k 0.7..1.0 (0.6..0.8) | 37.7k 0.8..1.3 (0.7..0.9)
+// From 10^6 rays on, strips where they are set below: tiled 1.2..1.8, in random
+// order 0.9..1.0 (bucket 20) and 0.8 (bucket 5).
+struct ForceRule {
+  size_t shared;
+  bool strips;
+};
+ForceRule force_rule(const TreeDev &T, double theta) {
+  const bool full = T.nparticles >= 4 * (long long)T.nnodes;  // buckets of 20: 7 particles a node, of 5: 1.9
+  if (T.periodic) return {0, false};
+  const bool narrow = theta < 0.15, wide = theta >= 0.25;
+  if (T.nnodes <= (full ? (narrow ? 1 << 16 : 1 << 12) : (wide ? 0 : 1 << 14))) return {(size_t)1 << 20, true};
+  if (full && (narrow || (!wide && T.nnodes <= 1 << 16))) return {(size_t)1 << 18, false};
+  return {(size_t)1 << 16, false};
+}
 
 // Whether a plane step of n rays walks two rays per lane.  A wave of the
 // one-ray kernel (5 blocks of 128 rays an SM) takes about 5.4 time units where
@@ -1939,9 +1974,10 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
     return 0;
   }
   (void)cudaGetLastError();
-  if (precision == GLB_PREC_FP64 && !t->tree->dev.periodic) {
+  const ForceRule rule = force_rule(t->tree->dev, t->tree->theta);
+  if (precision == GLB_PREC_FP64) {
     PartArgs p;
-    p.nparts = strip_parts(n, kPlanePartsMax, t->tree->dev.nnodes, &p.len);
+    p.nparts = strip_parts(n, rule.shared, t->tree->dev.nnodes, &p.len);
     // (in a capture the scratch would become the graph's: one launch, unshared)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (p.nparts > 1) CKR(cudaStreamIsCapturing(s, &cap));
@@ -1965,8 +2001,10 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
       return 0;
     }
   }
-  if (precision == GLB_PREC_FP64)
+  if (precision == GLB_PREC_FP64 && rule.strips)
     k_tree_force_f64<<<nblk(n, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
+  else if (precision == GLB_PREC_FP64)
+    k_tree_force<<<nblk(n, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
   else if (precision == GLB_PREC_SPLIT && !t->tree->dev.periodic && n >= kTwoRayMin && t->tree->theta < 0.2)
     k_tree_force_split2<<<nblk((n + 1) / 2, 128), 128, 0, s>>>(t->tree->dev, n, rays_dev, out_dev);
   else if (precision == GLB_PREC_SPLIT)

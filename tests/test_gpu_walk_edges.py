@@ -232,7 +232,7 @@ def test_device_forces_of_several_threads_and_sizes():
 
 def test_a_captured_device_force_is_one_unshared_launch():
     import torch
-    t = glb.TreeQuadParticles(_cluster(13, 20000), bucket=5, theta_force=0.1)
+    t = glb.TreeQuadParticles(_cluster(13, 60000), bucket=5, theta_force=0.1)
     x = np.random.default_rng(14).normal(0, 0.3, (1 << 16, 2))
     want = _device_force(t, x)[:300]
     d = torch.from_numpy(x[:300].copy()).cuda()
@@ -302,3 +302,28 @@ def test_a_refused_allocation_takes_back_the_unused_scratch():
         _refused(lambda: lens.rayshooterInternal(np.zeros((60000, 2))))
     assert torch.cuda.mem_get_info()[0] >= free + (64 << 20)
     assert np.array_equal(_recur(t, x), want)
+
+
+@pytest.mark.parametrize("n,bucket,theta,limit", [
+    (20000, 5, 0.1, 1 << 20), (20000, 20, 0.3, 1 << 20), (60000, 20, 0.1, 1 << 20),  # by strips from there on
+    (60000, 20, 0.2, 1 << 18), (600000, 20, 0.1, 1 << 18),                            # node by node
+    (60000, 5, 0.1, 1 << 16), (20000, 5, 0.3, 1 << 16), (60000, 20, 0.3, 1 << 16),
+])
+def test_device_forces_on_both_sides_of_their_limit(n, bucket, theta, limit):
+    t = glb.TreeQuadParticles(_cluster(n + bucket, n), bucket=bucket, theta_force=theta, inv_screening_scale=1.0)
+    x = np.random.default_rng(22).normal(0, 0.3, (limit, 2))
+    few = _device_force(t, x[:3000])
+    assert np.array_equal(_device_force(t, x[:2999]), few[:2999])
+    for m in (limit - 1, limit):
+        got = _device_force(t, x[:m])
+        assert np.all(np.isfinite(got))
+        assert np.all(np.abs(got[:3000] - few).max(axis=0) <= 1e-11 * np.abs(few).max(axis=0))
+
+
+@pytest.mark.parametrize("n", [1, 100, 70000])
+def test_periodic_device_forces(n):
+    t = glb.TreeQuadParticles(_cluster(23, 900), bucket=5, theta_force=0.1, periodic_buffer=True,
+                              inv_screening_scale=1.0)
+    x = np.random.default_rng(24).normal(0, 0.3, (n, 2))
+    want = _recur(t, x)[:, :5]
+    assert np.all(np.abs(_device_force(t, x) - want).max(axis=0) <= 1e-11 * np.abs(want).max(axis=0))
