@@ -1455,9 +1455,16 @@ int strip_parts(size_t n, size_t max_rays, int nnodes, int *len) {
   *len = (int)(per * kCutStep);
   return (int)((cuts + per - 1) / per);
 }
-// Plane steps share walks below this many rays; from here on a call has a warp
-// for every slot of the GPU by itself.
-constexpr size_t kPlanePartsMax = (size_t)1 << 16;
+// Plane steps share walks below this many rays: 2^16, where a call has a warp
+// for every slot of the GPU by itself, or as many rays as the tree has nodes.
+// Fewer rays than nodes are far apart, so that walks are long and uneven, and the
+// longest of a wave or two decide.  One plane, FP64, ms unshared / shared (rays
+// over 10 and 90 arcsec): 102,400 rays, 144k nodes 6.4 / 5.8, 13.3 / 8.1; 289k
+// nodes 9.2 / 7.8, 21.3 / 12.6; 262,144 rays, 289k nodes 14.4 / 15.5, 20.9 / 16.3;
+// 579k nodes 19.9 / 19.2, 32.4 / 23.3.  With more rays than nodes the two-ray
+// kernel is the better one: 262,144 rays, 144k nodes 11.0 / 12.3, 14.2 / 12.3,
+// 38k nodes 6.6 / 7.6.
+size_t plane_parts_max(int nnodes) { return std::max((size_t)1 << 16, std::min((size_t)nnodes, (size_t)1 << 20)); }
 // Host tree forces likewise (one walk per ray, so that a last, partly filled
 // wave weighs more than in a lens's planes).
 constexpr size_t kForcePartsMax = (size_t)1 << 18;
@@ -1553,7 +1560,7 @@ size_t parts_sums(const glb_lens *l, size_t n, int precision) {
   for (size_t j = 0; j < l->planes.size(); ++j)
     if (const glb_halo *ph = single_tree(l, (int)j)) {
       int len;
-      const int parts = strip_parts(n, kPlanePartsMax, ph->tree->dev.nnodes, &len);
+      const int parts = strip_parts(n, plane_parts_max(ph->tree->dev.nnodes), ph->tree->dev.nnodes, &len);
       if (parts > 1) m = std::max(m, (size_t)parts * 5 * n * sizeof(double));
     }
   return m;
@@ -1591,7 +1598,7 @@ int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int prec
     if (scratch && j % kPartCounters == 0) CKR(cudaMemsetAsync(scratch + sums, 0, kPartCounters * sizeof(int), s));
     if (scratch && !d_counts && precision == GLB_PREC_FP64 && !l->has_nfw && ptree) {
       PartArgs p;
-      p.nparts = strip_parts(n, kPlanePartsMax, a.tree.nnodes, &p.len);
+      p.nparts = strip_parts(n, plane_parts_max(a.tree.nnodes), a.tree.nnodes, &p.len);
       if (p.nparts > 1) {
         p.px = a.st;
         p.py = a.st + n;
@@ -1671,7 +1678,7 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
   }
   if (int rc = upload_lens(l)) return rc;
   if (int rc = ensure_ws(w, n, zs != nullptr)) return rc;
-  // shared walks: calls below kPlanePartsMax rays, which run in one slab;
+  // shared walks (plane_parts_max: calls of one slab);
   // without memory for their scratch the walks are not shared
   size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
   ABuf<char> parts(s);

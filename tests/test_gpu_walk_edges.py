@@ -327,3 +327,22 @@ def test_periodic_device_forces(n):
     x = np.random.default_rng(24).normal(0, 0.3, (n, 2))
     want = _recur(t, x)[:, :5]
     assert np.all(np.abs(_device_force(t, x) - want).max(axis=0) <= 1e-11 * np.abs(want).max(axis=0))
+
+
+def test_lens_calls_with_fewer_rays_than_nodes():
+    """One plane of 100,000 nodes: calls on both sides of that many rays share
+    and do not share their walks, and agree."""
+    p = _cluster(25, 700000, 0.001)
+    p["Mass"] *= 1e9
+    lens = glb.Lens(2.0)
+    lens.insertMainHalo(glb.LensHaloParticles(p, 0.3), True)
+    x = np.random.default_rng(26).normal(0, 60 * synth.ARCSEC, (130000, 2))
+    zs = np.random.default_rng(27).uniform(0.1, 3.0, len(x))
+    for z in (None, zs):
+        want = lens.rayshooterInternal(x[:65535], None if z is None else z[:65535])
+        for n in (65536, 80000, 130000):
+            y, A = lens.rayshooterInternal(x[:n], None if z is None else z[:n])
+            assert np.abs(y[:65535] - want[0]).max() < 1e-11 * np.abs(want[0]).max()
+            assert np.abs(A[:65535] - want[1]).max() < 1e-8 * np.abs(want[1]).max()
+            got = _noalloc(lens, x[:n]) if n <= 65536 and z is None else (y, A)
+            assert np.abs(got[0] - y).max() < 1e-11 * np.abs(y).max()
