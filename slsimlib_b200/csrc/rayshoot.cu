@@ -418,7 +418,7 @@ __device__ __forceinline__ void particle_halo_acc(const TreeDev &T, double rx, d
                                                   WalkCount *wc = nullptr) {
   auto walk = [&](double x, double y) {
     if (PREC == GLB_PREC_FP64)
-      walk_f64<COUNT>(T, x, y, valid, acc, wc);
+      walk_f64<false, COUNT>(T, x, y, valid, acc, wc);
     else if (PREC == GLB_PREC_FP32)
       walk_split<true>(T, x, y, valid, acc);
     else
@@ -1126,6 +1126,21 @@ __global__ void __launch_bounds__(128, 4) k_tree_force_phi(const __grid_constant
   particle_halo_f64<true>(T, valid ? px[k] : 0.0, valid ? py[k] : 0.0, valid, S.warp[t >> 5], S.tab, acc, 1);
   if (valid) out.put(perm[k], acc);
 }
+// The same node by node (host_force_rule).
+__global__ void __launch_bounds__(128) k_tree_force_phi_node(const __grid_constant__ TreeDev T, size_t n,
+                                                            const double *px, const double *py, const unsigned *perm,
+                                                            ForceOut out) {
+  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const bool valid = k < n;
+  if (!__any_sync(kFull, valid)) return;
+  const double rx = valid ? px[k] : 0.0, ry = valid ? py[k] : 0.0;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  const int im = T.periodic ? 1 : 0;
+  for (int i = -im; i <= im; ++i)
+    for (int j = -im; j <= im; ++j)
+      walk_f64<true>(T, im ? rx + i * T.period_x : rx, im ? ry + j * T.period_y : ry, valid, acc);
+  if (valid) out.put(perm[k], acc);
+}
 __global__ void __launch_bounds__(32 * kSumRows) k_force_parts_end(const __grid_constant__ TreeDev T, size_t n,
                                                                   const double *part, const unsigned char *used,
                                                                   int nparts, const unsigned *perm, ForceOut out) {
@@ -1465,9 +1480,6 @@ int strip_parts(size_t n, size_t max_rays, int nnodes, int *len) {
 // kernel is the better one: 262,144 rays, 144k nodes 11.0 / 12.3, 14.2 / 12.3,
 // 38k nodes 6.6 / 7.6.
 size_t plane_parts_max(int nnodes) { return std::max((size_t)1 << 16, std::min((size_t)nnodes, (size_t)1 << 20)); }
-// Host tree forces likewise (one walk per ray, so that a last, partly filled
-// wave weighs more than in a lens's planes).
-constexpr size_t kForcePartsMax = (size_t)1 << 18;
 // FP64 forces at device positions: shared below `shared` rays; from there on, or
 // where they cannot be shared, by strips or node by node.  The rays come in the
 // caller's order, so a warp's may lie anywhere; then, and where leaves hold few
@@ -1497,6 +1509,25 @@ ForceRule force_rule(const TreeDev &T, double theta) {
   if (T.nnodes <= (full ? (narrow ? 1 << 16 : 1 << 12) : (wide ? 0 : 1 << 14))) return {(size_t)1 << 20, true};
   if (full && (narrow || (!wide && T.nnodes <= 1 << 16))) return {(size_t)1 << 18, false};
   return {(size_t)1 << 16, false};
+}
+// The same for host positions, sorted along a Morton curve, with the potential.
+// Times, ms, shared / strips / node by node, 2.5e5 rays over 20 arcsec:
+//   angle 0.1, bucket 5: 10.8k nodes 7.2 / 8.2 / 10.7, 141k 13.8 / 16.2 / 14.4,
+//   539k 17.9 / 21.6 / 16.8, 2.15M 23.9 / 28.8 / 20.6; bucket 20: 37.7k 11.4 / 13.4 /
+//   15.8, 145k 15.5 / 18.6 / 17.5, 579k 21.1 / 25.5 / 21.1;
+//   angle 0.3, bucket 5: 10.8k 1.64 / 1.71 / 1.60, 141k 2.69 / 2.99 / 2.16, 2.15M 5.6 /
+//   6.1 / 4.2; bucket 20: 37.7k 2.47 / 2.77 / 2.23, 579k 5.1 / 5.6 / 4.0.
+// 1.2e5 rays: shared by 1.1 to 1.4 at angle 0.1 except bucket 5 from 539k nodes on
+// (equal to 1.2 slower), slower by 1.05 to 1.4 at 0.3; 60,000 rays: shared within
+// 0.9..1.5 everywhere.  10^6 rays: strips before node by node below 2^16 nodes at
+// angle 0.1 (1.1 to 1.3), behind it (1.0 to 1.5) elsewhere.
+ForceRule host_force_rule(const TreeDev &T, double theta) {
+  const ForceRule r = force_rule(T, theta);
+  const bool full = T.nparticles >= 4 * (long long)T.nnodes;
+  if (theta < 0.15)
+    return {T.periodic ? 0 : (size_t)1 << (full || T.nnodes <= 1 << 18 ? 18 : 17), T.nnodes <= 1 << 16};
+  if (T.periodic) return {0, T.nnodes <= 1 << 12};
+  return {(size_t)1 << (r.strips ? 18 : theta < 0.25 ? 17 : 16), r.strips};
 }
 
 // Whether a plane step of n rays walks two rays per lane.  A wave of the
@@ -1842,10 +1873,11 @@ int glb_tree_destroy(glb_tree *t) {
 // pool's: a buffer kept on the tree would have to be that large, and one
 // allocated for each call cost 2 to 5 ms of a 1.5 ms call (3,000 rays, opening
 // angle 0.3).
-static int force_particles(const TreeDev &T, cudaStream_t s, size_t n, const double *xcm, double *alpha, double *kappa,
-                           double *gamma, double *phi) {
+static int force_particles(const TreeDev &T, double theta, cudaStream_t s, size_t n, const double *xcm, double *alpha,
+                           double *kappa, double *gamma, double *phi) {
   PartArgs p;
-  p.nparts = T.periodic ? 1 : strip_parts(n, kForcePartsMax, T.nnodes, &p.len);
+  const ForceRule rule = host_force_rule(T, theta);
+  p.nparts = strip_parts(n, rule.shared, T.nnodes, &p.len);
   size_t tb = 0;
   CKR(cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned *)nullptr, (unsigned *)nullptr, (unsigned *)nullptr,
                                       (unsigned *)nullptr, (int)n, 0, 32, s));
@@ -1889,8 +1921,10 @@ static int force_particles(const TreeDev &T, cudaStream_t s, size_t n, const dou
     CKR(cudaMemsetAsync(p.counter, 0, sizeof(int), s));
     if (int rc = launch_parts<true>(T, p, s)) return rc;
     k_force_parts_end<<<nblk(n, 32), dim3(32, kSumRows), 0, s>>>(T, n, p.out, p.used, p.nparts, perm, fo);
-  } else {
+  } else if (rule.strips) {
     k_tree_force_phi<<<nblk(n, 128), 128, 0, s>>>(T, n, px, py, perm, fo);
+  } else {
+    k_tree_force_phi_node<<<nblk(n, 128), 128, 0, s>>>(T, n, px, py, perm, fo);
   }
   CKR(cudaGetLastError());
   if (alpha) CKR(cudaMemcpyAsync(alpha, fo.alpha, 2 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1901,7 +1935,7 @@ static int force_particles(const TreeDev &T, cudaStream_t s, size_t n, const dou
   return 0;
 }
 
-static int force_generic(const HaloDev &H, int device, cudaStream_t s, size_t n, const double *xcm, double *alpha,
+static int force_generic(const HaloDev &H, double theta, int device, cudaStream_t s, size_t n, const double *xcm, double *alpha,
                          double *kappa, double *gamma, double *phi, int subtract = 0, double screening = 1.0) {
   if (n == 0) return 0;
   if (!xcm) return fail(GLB_ERR_ARG, "null positions");
@@ -1911,7 +1945,7 @@ static int force_generic(const HaloDev &H, int device, cudaStream_t s, size_t n,
     for (size_t o = 0; o < n;) {
       const size_t m = std::min(chunk, n - o);
       const int rc =
-          force_particles(H.tree, s, m, xcm + 2 * o, alpha ? alpha + 2 * o : nullptr, kappa ? kappa + o : nullptr,
+          force_particles(H.tree, theta, s, m, xcm + 2 * o, alpha ? alpha + 2 * o : nullptr, kappa ? kappa + o : nullptr,
                           gamma ? gamma + 3 * o : nullptr, phi ? phi + o : nullptr);
       if (rc == GLB_ERR_OOM && m > 65536) {
         chunk = m / 2;
@@ -1966,7 +2000,7 @@ int glb_tree_force2D_recur(glb_tree *t, size_t n, const double *rays, double *al
     }
     return 0;
   }
-  return force_generic(H, t->device, t->stream, n, rays, alpha, kappa, gamma, phi);
+  return force_generic(H, t->tree->theta, t->device, t->stream, n, rays, alpha, kappa, gamma, phi);
 }
 
 int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double *out_dev, int precision,
@@ -2266,7 +2300,7 @@ int glb_halo_force_ex(glb_halo *h, size_t n, const double *xcm, double *alpha, d
     }
     return 0;
   }
-  int rc = force_generic(H, h->device, h->stream, n, xcm, alpha, kappa, gamma, phi, subtract_point, screening);
+  int rc = force_generic(H, h->tree ? h->tree->theta : 0.0, h->device, h->stream, n, xcm, alpha, kappa, gamma, phi, subtract_point, screening);
   if (rc) return rc;
   if (h->kind == HALO_PARTICLES && alpha)  // LensHaloParticles::force_halo negates alpha
     for (size_t i = 0; i < 2 * n; ++i) alpha[i] = -alpha[i];

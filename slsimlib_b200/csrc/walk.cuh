@@ -57,12 +57,13 @@ __device__ __forceinline__ void bspline_f64(double x0, double x1, double r, doub
   if (PHI) acc[5] -= Mass * log(r) / kPi;
 }
 
-// One warp-synchronous walk for the ray (rx, ry), node by node: the form that
-// counts interactions (walk_strip.cuh computes the FP64 forces).  Lanes that
-// are not `valid` take part in the votes but add nothing.  acc = {alpha0,
-// alpha1, kappa, gamma0, gamma1} accumulates in the reference's units (alpha
+// One warp-synchronous walk for the ray (rx, ry), node by node: lenses with NFW
+// haloes, tree forces where strips are slower (force_rule, host_force_rule) and
+// the count of interactions; the other FP64 forces take walk_strip.cuh.  Lanes
+// that are not `valid` take part in the votes but add nothing.  acc = {alpha0,
+// alpha1, kappa, gamma0, gamma1, phi} accumulates in the reference's units (alpha
 // pointing away from mass).
-template <bool COUNT>
+template <bool PHI, bool COUNT = false>
 __device__ __forceinline__ void walk_f64(const TreeDev &T, double rx, double ry, bool valid, double *acc,
                                          WalkCount *wc = nullptr) {
   const double inv_pi = 1.0 / kPi;
@@ -92,12 +93,17 @@ __device__ __forceinline__ void walk_f64(const TreeDev &T, double rx, double ry,
       tmp = -2.0 * mass * inv_pi * ir4 * scr;
       acc[3] += 0.5 * (dx * dx - dy * dy) * tmp;
       acc[4] += dx * dy * tmp;
+      if (PHI) {
+        acc[5] += 0.5 * T.phi_mass * log(r2) * inv_pi * scr;
+        acc[5] -= 0.5 * (T.phi_q0 * dx * dx + T.phi_q1 * dy * dy + 2 * T.phi_q2 * dx * dy) * inv_pi * ir4 * scr;
+      }
       acc[0] -= (q0 * dx + q2 * dy) * ir4 * inv_pi * scr;
       acc[1] -= (q1 * dy + q2 * dx) * ir4 * inv_pi * scr;
       tmp = 4 * (q0 * dx * dx + q1 * dy * dy + 2 * q2 * dx * dy) * (ir4 / r2) * inv_pi * scr;
       acc[0] += tmp * dx;
       acc[1] += tmp * dy;
       acc[2] -= T.inv_area * mass;
+      if (PHI) acc[5] -= 0.5 * mass * r2 * T.inv_area;
       resume = skip;
     }
     if (!__any_sync(kFull, open)) {
@@ -126,13 +132,14 @@ __device__ __forceinline__ void walk_f64(const TreeDev &T, double rx, double ry,
           acc[3] += 0.5 * (x0 * x0 - x1 * x1) * tmp;
           acc[4] += x0 * x1 * tmp;
           acc[2] -= m * T.inv_area;
+          if (PHI) acc[5] += prefac * rcm2 * 0.5 * log(rcm2) - m * T.inv_area * rcm2 / 2;
           if (COUNT) wc->P++;
           // the leaf's big particles are those smaller than the leaf (quadTree.h:384-395)
           const double size = (double)P.w;
           if (COUNT && nearc && size < width) wc->B++;
           if (nearc && size < width && rcm2 < 4 * size * size) {
             if (COUNT) wc->S++;
-            bspline_f64<false>(x0, x1, sqrt(rcm2), m, size, T.phiintconst, acc);
+            bspline_f64<PHI>(x0, x1, sqrt(rcm2), m, size, T.phiintconst, acc);
           }
         }
       }
@@ -150,7 +157,7 @@ __device__ __forceinline__ void walk_f64(const TreeDev &T, double rx, double ry,
             if (COUNT) wc->B++;
             if (rcm2 < 4 * size * size) {
               if (COUNT) wc->S++;
-              bspline_f64<false>(x0, x1, sqrt(rcm2), (double)P.z, size, T.phiintconst, acc);
+              bspline_f64<PHI>(x0, x1, sqrt(rcm2), (double)P.z, size, T.phiintconst, acc);
             }
           }
         }

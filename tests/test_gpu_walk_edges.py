@@ -346,3 +346,35 @@ def test_lens_calls_with_fewer_rays_than_nodes():
             assert np.abs(A[:65535] - want[1]).max() < 1e-8 * np.abs(want[1]).max()
             got = _noalloc(lens, x[:n]) if n <= 65536 and z is None else (y, A)
             assert np.abs(got[0] - y).max() < 1e-11 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("n,bucket,theta,kw,limit", [
+    (20000, 5, 0.1, {}, 1 << 18), (600000, 5, 0.1, {}, 1 << 17), (20000, 20, 0.3, dict(inv_area=0.1), 1 << 18),
+    (60000, 20, 0.2, dict(inv_area=0.1), 1 << 17), (60000, 5, 0.3, dict(inv_screening_scale=1.0, inv_area=0.2), 1 << 16),
+])
+def test_host_forces_on_both_sides_of_their_limit(n, bucket, theta, kw, limit):
+    t = glb.TreeQuadParticles(_cluster(n + bucket, n), bucket=bucket, theta_force=theta, **kw)
+    x = np.random.default_rng(28).normal(0, 0.3, (limit, 2))
+    few = _recur(t, x[:3000])
+    for m in (limit - 1, limit):
+        got = _recur(t, x[:m])
+        assert np.all(np.isfinite(got))
+        assert np.all(np.abs(got[:3000] - few).max(axis=0) <= 1e-11 * np.abs(few).max(axis=0))
+    assert np.all(np.abs(_device_force(t, x[:3000]) - few[:, :5]).max(axis=0) <= 1e-11 * np.abs(few[:, :5]).max(axis=0))
+
+
+@pytest.mark.parametrize("np_,theta", [(700, 0.1), (30000, 0.3)])
+def test_node_by_node_potential_matches_the_oracle(np_, theta):
+    from tests import harness as H
+    from tests.test_gpu_parity import force_err, pack
+    p = _cluster(np_, np_, 0.02)
+    x = np.random.default_rng(29).normal(0, 0.3, (70000, 2))
+    x[0] = p["x"][0, :2]
+    for periodic in (False, True):
+        if periodic and np_ > 1000:
+            continue
+        t = glb.TreeQuadParticles(p, bucket=5, theta_force=theta, inv_screening_scale=1.0, periodic_buffer=periodic)
+        o = H.OracleTree(p, bucket=5, theta=theta, inv_area=0.0, inv_screening=1.0, periodic=int(periodic))
+        got = pack(*t.force2D_recur(x))[:257]
+        err, cols = force_err(got, o.force(x[:257]))
+        assert err < 1e-9, cols
