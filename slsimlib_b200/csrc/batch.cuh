@@ -55,20 +55,22 @@ constexpr int kBatchSmemDoubles = 22;
 // The kernel's form.  FP64: GLB_PREC_FP64 (the node-at-a-time walk: batches with
 // NFW haloes, see launch_plane_steps) or kStripForm (the strip walk: every other
 // batch).  Split: kListForm (the list walk) or, for batches with a tree of more
-// than kListMaxNodes nodes, GLB_PREC_SPLIT (the node-at-a-time walk): where a
+// nodes than list_max_nodes, GLB_PREC_SPLIT (the node-at-a-time walk): where a
 // warp's rays are spread over several leaves, most cells near the opening radius
-// are mixed.  One plane, 512^2 rays over 30 arcsec, node by node / list, ms: 2^16
-// particles 6.5 / 3.8, 2^18 7.8 / 4.8, 2^20 (151,000 nodes) 9.9 / 9.1, 2^22
-// (604,000) 16.7 / 22.1; over 600 arcsec 2^20 18.9 / 17.7, 2^22 62.5 / 59.2.
+// are mixed.  One plane, node by node / list, ms: 72,000 nodes, 8 lenses of 300^2
+// rays over 30 arcsec 22.7 / 17.3, 32 of 96^2 14.1 / 13.3; 144,000 nodes 26.9 / 30.2
+// and 20.5 / 26.0.  Few rays leave warps idle, and the shorter chain of the list
+// walk counts: 144,000 nodes, 8 of 64^2 13.0 / 11.7, 8 of 128^2 11.6 / 11.6; 604,000
+// nodes, 512^2 16.7 / 22.1.
 constexpr int kStripForm = 3, kListForm = 4;
-constexpr int kListMaxNodes = 200000;
-int batch_form(const std::vector<glb_lens *> &lenses, int precision) {
+int list_max_nodes(size_t rays) { return rays <= (size_t)1 << 17 ? 200000 : 100000; }
+int batch_form(const std::vector<glb_lens *> &lenses, int precision, size_t rays) {
   for (const glb_lens *l : lenses) {
     if (precision == GLB_PREC_FP64 && l->has_nfw) return GLB_PREC_FP64;
     if (precision == GLB_PREC_SPLIT)
       for (const PlaneHost *p : l->planes)
         for (const glb_halo *h : p->halos)
-          if (h->tree && h->tree->dev.nnodes > kListMaxNodes) return GLB_PREC_SPLIT;
+          if (h->tree && h->tree->dev.nnodes > list_max_nodes(rays)) return GLB_PREC_SPLIT;
   }
   return precision == GLB_PREC_SPLIT ? kListForm : kStripForm;
 }
@@ -446,7 +448,7 @@ int glb_batch_create_grids(glb_lens *const *lenses, int nlens, const size_t *n1d
   CKR(cudaMemcpy(b->d_lenses.p, L.data(), nlens * sizeof(LensDev), cudaMemcpyHostToDevice));
   if (int rc = batch_chunks(b.get(), 3)) return rc;
   if (int rc = device_nfw_tables(b->tab)) return rc;
-  b->form = batch_form(b->lenses, precision);
+  b->form = batch_form(b->lenses, precision, b->total);
   if (int rc = persistent_grid(b->block, b->form, &b->grid)) return rc;
   *out = b.release();
   return 0;
@@ -1004,7 +1006,7 @@ int glb_server_create(glb_lens *const *models, int nmodels, size_t max_rays_per_
   CKR(S->d_lenses.alloc(nmodels));
   CKR(cudaMemcpy(S->d_lenses.p, L.data(), nmodels * sizeof(LensDev), cudaMemcpyHostToDevice));
   if (int rc = device_nfw_tables(S->tab)) return rc;
-  S->form = batch_form(S->models, precision);
+  S->form = batch_form(S->models, precision, S->cap);  // (a batch may hold so many)
   if (int rc = persistent_grid(128, S->form, &S->grid)) return rc;
   size_t cap = S->cap;
   for (int i = 0; i < nslots; ++i) {

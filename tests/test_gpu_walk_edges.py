@@ -378,3 +378,23 @@ def test_node_by_node_potential_matches_the_oracle(np_, theta):
         got = pack(*t.force2D_recur(x))[:257]
         err, cols = force_err(got, o.force(x[:257]))
         assert err < 1e-9, cols
+
+
+@pytest.mark.parametrize("sides", [(33,), (300, 300)])  # the list walk, and too many rays for it
+def test_split_batches_of_a_large_tree(sides):
+    """A tree of about 130,000 nodes in a split-form batch: every ray's result is
+    the lens path's of a plane with two particle haloes (a walk per ray)."""
+    p, q = _cluster(30, 900000, 0.001), _cluster(31, 40, 0.05)
+    for c in (p, q):
+        c["Mass"] *= 1e9
+    lens = glb.Lens(2.0)
+    for c in (p, q):
+        lens.insertMainHalo(glb.LensHaloParticles(c, 0.3), True)
+    rng = 100 * synth.ARCSEC
+    b = glb.GridBatch([lens] * len(sides), sides, [(0.0, 0.0)] * len(sides), [rng] * len(sides), glb.PREC_SPLIT)
+    b.run()
+    for i, side in enumerate(sides):
+        y, A = b.result(i)
+        g = glb.GridMap(lens, side, (0.0, 0.0), rng, glb.PREC_SPLIT)
+        assert np.abs(y - g.y).max() <= 1e-13 * np.abs(g.y).max()
+        assert np.abs(A - g.A).max() <= 1e-13 * np.abs(g.A).max()
