@@ -52,28 +52,27 @@ struct Chunk {
 // distinct banks).  Keeping them out of registers leaves the tree walk the
 // registers it needs.
 constexpr int kBatchSmemDoubles = 22;
-// The kernel's form.  FP64: GLB_PREC_FP64 (the node-at-a-time walk: batches with
-// NFW haloes, see launch_plane_steps) or kStripForm (the strip walk: every other
-// batch).  Split: kListForm (the list walk) or, for batches with a tree of more
-// nodes than list_max_nodes, GLB_PREC_SPLIT (the node-at-a-time walk): where a
-// warp's rays are spread over several leaves, most cells near the opening radius
-// are mixed.  One plane, node by node / list, ms: 72,000 nodes, 8 lenses of 300^2
+// The kernel's form for a lens (a batch has a launch for each form among its
+// lenses, so that no lens's results depend on the others).  FP64: GLB_PREC_FP64
+// (the node-at-a-time walk: lenses with NFW haloes, see launch_plane_steps) or
+// kStripForm (the strip walk: every other lens).  Split: kListForm (the list walk)
+// or, for lenses with a tree of more nodes than list_max_nodes, GLB_PREC_SPLIT
+// (the node-at-a-time walk, the same bits): where a warp's rays are spread over
+// several leaves, most cells near the opening radius are mixed.  One plane, node by node / list, ms: 72,000 nodes, 8 lenses of 300^2
 // rays over 30 arcsec 22.7 / 17.3, 32 of 96^2 14.1 / 13.3; 144,000 nodes 26.9 / 30.2
 // and 20.5 / 26.0.  Few rays leave warps idle, and the shorter chain of the list
 // walk counts: 144,000 nodes, 8 of 64^2 13.0 / 11.7, 8 of 128^2 11.6 / 11.6; 604,000
 // nodes, 512^2 16.7 / 22.1.
 constexpr int kStripForm = 3, kListForm = 4;
 int list_max_nodes(size_t rays) { return rays <= (size_t)1 << 17 ? 200000 : 100000; }
-int batch_form(const std::vector<glb_lens *> &lenses, int precision, size_t rays) {
-  for (const glb_lens *l : lenses) {
-    if (precision == GLB_PREC_FP64 && l->has_nfw) return GLB_PREC_FP64;
-    if (precision == GLB_PREC_SPLIT)
-      for (const PlaneHost *p : l->planes)
-        for (const glb_halo *h : p->halos)
-          if (h->tree && h->tree->dev.nnodes > list_max_nodes(rays)) return GLB_PREC_SPLIT;
-  }
-  return precision == GLB_PREC_SPLIT ? kListForm : kStripForm;
+int batch_form(const glb_lens *l, int precision, size_t rays) {
+  if (precision == GLB_PREC_FP64) return l->has_nfw ? GLB_PREC_FP64 : kStripForm;
+  for (const PlaneHost *p : l->planes)
+    for (const glb_halo *h : p->halos)
+      if (h->tree && h->tree->dev.nnodes > list_max_nodes(rays)) return GLB_PREC_SPLIT;
+  return kListForm;
 }
+constexpr int kForms = 5;
 // The exponential's tables: those of any particle tree in the batch.
 const ExpTab *batch_exptab(const std::vector<glb_lens *> &lenses) {
   for (const glb_lens *l : lenses)
@@ -318,9 +317,27 @@ int persistent_grid(int block, int form, int *grid) {
   return 0;
 }
 
-int launch_batch(int form, int grid, int block, cudaStream_t s, const Chunk *chunks, int nchunks,
-                 const LensDev *lenses, const NFWTables &tab, const double *xs, const unsigned *outidx, double *y,
-                 double *A, int *counter, const ExpTab *exptab) {
+// A batch's launches, one per form: consecutive chunks of lenses of that form.
+struct FormRuns {
+  int first[kForms + 1] = {0, 0, 0, 0, 0, 0};
+  int grid[kForms] = {0, 0, 0, 0, 0};
+};
+// Counts `chunks`, sorted by the forms of their lenses, into runs.
+void form_runs(const std::vector<Chunk> &chunks, const std::vector<int> &form, FormRuns &r) {
+  int n[kForms] = {0, 0, 0, 0, 0};
+  for (const Chunk &c : chunks) ++n[form[c.lens]];
+  for (int f = 0; f < kForms; ++f) r.first[f + 1] = r.first[f] + n[f];
+}
+int form_grids(const std::vector<int> &form, int block, FormRuns &r) {
+  for (int f = 0; f < kForms; ++f)
+    if (std::find(form.begin(), form.end(), f) != form.end())
+      if (int rc = persistent_grid(block, f, &r.grid[f])) return rc;
+  return 0;
+}
+
+int launch_form(int form, int grid, int block, cudaStream_t s, const Chunk *chunks, int nchunks,
+                const LensDev *lenses, const NFWTables &tab, const double *xs, const unsigned *outidx, double *y,
+                double *A, int *counter, const ExpTab *exptab) {
   const size_t smem = batch_smem_bytes(block, form);
   if (form == GLB_PREC_SPLIT)
     k_batch<GLB_PREC_SPLIT><<<grid, block, smem, s>>>(chunks, nchunks, lenses, tab, xs, outidx, y, A, counter, exptab);
@@ -337,22 +354,36 @@ int launch_batch(int form, int grid, int block, cudaStream_t s, const Chunk *chu
   return 0;
 }
 
+// counters: kForms integers on the device.
+int launch_batch(const FormRuns &r, int block, cudaStream_t s, const Chunk *chunks, const LensDev *lenses,
+                 const NFWTables &tab, const double *xs, const unsigned *outidx, double *y, double *A, int *counters,
+                 const ExpTab *exptab) {
+  CKR(cudaMemsetAsync(counters, 0, kForms * sizeof(int), s));
+  for (int f = 0; f < kForms; ++f)
+    if (const int n = r.first[f + 1] - r.first[f])
+      if (int rc = launch_form(f, r.grid[f], block, s, chunks + r.first[f], n, lenses, tab, xs, outidx, y, A,
+                               counters + f, exptab))
+        return rc;
+  return 0;
+}
+
 }  // namespace
 
 // ================================================================ batch plan
 struct glb_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
-  int form = GLB_PREC_FP64;  // k_batch's
-  int block = 128, grid = 0;
+  int block = 128;
   std::vector<glb_lens *> lenses;
+  std::vector<int> form;  // k_batch's, per lens
+  FormRuns runs;
+  const ExpTab *exptab = nullptr;
   std::vector<size_t> n1d, offset;
   std::vector<double> centers, ranges;
   int tile_log2w = 3;  // grid tiles of 8 x 4 rays (autotuned: 8 x 4, 16 x 2, 32 x 1)
   size_t total = 0;
   DBuf<LensDev> d_lenses;
   DBuf<Chunk> d_chunks;
-  int nchunks = 0;
   DBuf<double> y, A;
   DBuf<int> counter;
   NFWTables tab{};
@@ -389,10 +420,13 @@ int batch_chunks(glb_batch *b, int log2w) {
       }
   }
   if (C.size() > 0x7fffffffull) return fail(GLB_ERR_ARG, "too many chunks");
-  std::stable_sort(C.begin(), C.end(), [&](const Chunk &x, const Chunk &y) { return x.n1d > y.n1d; });
+  std::stable_sort(C.begin(), C.end(), [&](const Chunk &x, const Chunk &y) {
+    const int fx = b->form[x.lens], fy = b->form[y.lens];
+    return fx != fy ? fx < fy : x.n1d > y.n1d;
+  });
+  form_runs(C, b->form, b->runs);
   if (b->d_chunks.n < C.size()) CKR(b->d_chunks.alloc(C.size()));
   CKR(cudaMemcpy(b->d_chunks.p, C.data(), C.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
-  b->nchunks = (int)C.size();
   b->tile_log2w = log2w;
   return 0;
 }
@@ -408,9 +442,8 @@ void drop_graph(glb_batch *b) {
 
 int batch_enqueue(glb_batch *b) {
   (void)cudaGetLastError();  // launch errors below are this launch's own
-  CKR(cudaMemsetAsync(b->counter.p, 0, sizeof(int), b->stream));
-  return launch_batch(b->form, b->grid, b->block, b->stream, b->d_chunks.p, b->nchunks, b->d_lenses.p, b->tab, nullptr,
-                      nullptr, b->y.p, b->A.p, b->counter.p, batch_exptab(b->lenses));
+  return launch_batch(b->runs, b->block, b->stream, b->d_chunks.p, b->d_lenses.p, b->tab, nullptr, nullptr, b->y.p,
+                      b->A.p, b->counter.p, b->exptab);
 }
 }  // namespace
 
@@ -444,12 +477,13 @@ int glb_batch_create_grids(glb_lens *const *lenses, int nlens, const size_t *n1d
   CKR(b->d_lenses.alloc(nlens));
   CKR(b->y.alloc(2 * b->total));
   CKR(b->A.alloc(4 * b->total));
-  CKR(b->counter.alloc(1));
+  CKR(b->counter.alloc(kForms));
   CKR(cudaMemcpy(b->d_lenses.p, L.data(), nlens * sizeof(LensDev), cudaMemcpyHostToDevice));
+  for (const glb_lens *l : b->lenses) b->form.push_back(batch_form(l, precision, b->total));
+  b->exptab = batch_exptab(b->lenses);
   if (int rc = batch_chunks(b.get(), 3)) return rc;
   if (int rc = device_nfw_tables(b->tab)) return rc;
-  b->form = batch_form(b->lenses, precision, b->total);
-  if (int rc = persistent_grid(b->block, b->form, &b->grid)) return rc;
+  if (int rc = form_grids(b->form, b->block, b->runs)) return rc;
   *out = b.release();
   return 0;
 }
@@ -499,20 +533,19 @@ int glb_batch_autotune(glb_batch *b, int *best_block, double *best_ms) {
     return 0;
   };
   double best = 1e300;
-  int bb = b->block, bg = b->grid;
+  int bb = b->block;
   for (int c : {64, 128, 256}) {
     b->block = c;
-    if (int rc = persistent_grid(c, b->form, &b->grid)) return rc;
+    if (int rc = form_grids(b->form, c, b->runs)) return rc;
     double t;
     if (int rc = time_it(&t)) return rc;
     if (t < best) {
       best = t;
       bb = c;
-      bg = b->grid;
     }
   }
   b->block = bb;
-  b->grid = bg;
+  if (int rc = form_grids(b->form, bb, b->runs)) return rc;
   int bt = b->tile_log2w;
   for (int w : {3, 4, 5}) {
     if (w == bt) continue;
@@ -548,7 +581,7 @@ int glb_batch_set_block(glb_batch *b, int block) {
   if (!b || (block != 64 && block != 128 && block != 256)) return fail(GLB_ERR_ARG, "block must be 64, 128 or 256");
   if (int rc = set_dev(b->device)) return rc;
   b->block = block;
-  if (int rc = persistent_grid(block, b->form, &b->grid)) return rc;
+  if (int rc = form_grids(b->form, block, b->runs)) return rc;
   drop_graph(b);
   return 0;
 }
@@ -667,7 +700,10 @@ struct Slot {
 struct glb_server {
   int device = 0;
   int precision = GLB_PREC_FP64;
-  int form = GLB_PREC_FP64;  // k_batch's
+  std::vector<int> form;  // k_batch's, per model
+  FormRuns runs;          // (grids; the launches are each batch's own)
+  bool mixed = false;     // the models' forms differ
+  const ExpTab *exptab = nullptr;
   size_t cap = 0;  // rays per batch at most (max_rays_per_batch; the pinned staging of a slot)
   size_t reserve = 0;  // device bytes admission leaves free for everything else
   size_t total_bytes = 0;
@@ -679,7 +715,6 @@ struct glb_server {
   std::vector<LensDev> h_lenses;  // host copies (source-plane defaults of each model)
   DBuf<LensDev> d_lenses;
   NFWTables tab{};
-  int grid = 0;
   std::vector<std::unique_ptr<Slot>> slots;
   std::mutex mu;
   std::condition_variable cv_submit, cv_done;
@@ -796,6 +831,9 @@ int launch_slot(glb_server *S, Slot &sl) {
       C.push_back(k);
     }
   }
+  if (S->mixed)
+    std::stable_sort(C.begin(), C.end(),
+                     [S](const Chunk &x, const Chunk &y) { return S->form[x.lens] < S->form[y.lens]; });
   int bits = 32;
   while ((1ull << (bits - 32)) < nr + 1 && bits < 64) ++bits;
   size_t tb = 0;
@@ -815,7 +853,7 @@ int launch_slot(glb_server *S, Slot &sl) {
   unsigned long long *keys = (unsigned long long *)(m + o_k), *keys2 = (unsigned long long *)(m + o_k2);
   unsigned *idx = (unsigned *)(m + o_idx), *perm = (unsigned *)(m + o_perm), *req_of = (unsigned *)(m + o_req);
   Chunk *dch = (Chunk *)(m + o_ch);
-  int *counter = (int *)(m + o_cnt);
+  int *counters = (int *)(m + o_cnt);
   CKR(cudaMemcpyAsync(dx, sl.hx, 2 * n * sizeof(double), cudaMemcpyHostToDevice, s));
   CKR(cudaMemcpyAsync(req_of, sl.hreq, n * sizeof(unsigned), cudaMemcpyHostToDevice, s));
   CKR(cudaMemcpyAsync(dbb, bb.data(), bb.size() * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -824,12 +862,10 @@ int launch_slot(glb_server *S, Slot &sl) {
   k_gather_sorted<<<nblk(n, 256), 256, 0, s>>>(dx, perm, n, dxs);
   // chunks: requests stay contiguous in sorted order; 32 rays per chunk
   CKR(cudaMemcpyAsync(dch, C.data(), C.size() * sizeof(Chunk), cudaMemcpyHostToDevice, s));
-  CKR(cudaMemsetAsync(counter, 0, sizeof(int), s));
-  if (!C.empty()) {
-    if (int rc = launch_batch(S->form, S->grid, 128, s, dch, (int)C.size(), S->d_lenses.p, S->tab, dxs, perm, dy, dA,
-                              counter, batch_exptab(S->models)))
-      return rc;
-  }
+  FormRuns runs = S->runs;
+  form_runs(C, S->form, runs);
+  if (int rc = launch_batch(runs, 128, s, dch, S->d_lenses.p, S->tab, dxs, perm, dy, dA, counters, S->exptab))
+    return rc;
   // large requests: the lens path's per-plane kernels over the request's rays
   // (contiguous in sorted order), results scattered to their batch slots
   double *st = (double *)(m + o_st);
@@ -1006,8 +1042,10 @@ int glb_server_create(glb_lens *const *models, int nmodels, size_t max_rays_per_
   CKR(S->d_lenses.alloc(nmodels));
   CKR(cudaMemcpy(S->d_lenses.p, L.data(), nmodels * sizeof(LensDev), cudaMemcpyHostToDevice));
   if (int rc = device_nfw_tables(S->tab)) return rc;
-  S->form = batch_form(S->models, precision, S->cap);  // (a batch may hold so many)
-  if (int rc = persistent_grid(128, S->form, &S->grid)) return rc;
+  for (const glb_lens *l : S->models) S->form.push_back(batch_form(l, precision, S->cap));  // (a batch may hold so many)
+  for (int f : S->form) S->mixed = S->mixed || f != S->form[0];
+  S->exptab = batch_exptab(S->models);
+  if (int rc = form_grids(S->form, 128, S->runs)) return rc;
   size_t cap = S->cap;
   for (int i = 0; i < nslots; ++i) {
     auto sl = std::make_unique<Slot>();

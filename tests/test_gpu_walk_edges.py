@@ -398,3 +398,46 @@ def test_split_batches_of_a_large_tree(sides):
         g = glb.GridMap(lens, side, (0.0, 0.0), rng, glb.PREC_SPLIT)
         assert np.abs(y - g.y).max() <= 1e-13 * np.abs(g.y).max()
         assert np.abs(A - g.A).max() <= 1e-13 * np.abs(g.A).max()
+
+
+def _mixed_lenses():
+    plain = [_lens(30000, 2), _lens(20000, 1)]
+    spec = synth.light_cone(seed=9, n_total=25000, n_planes=2, halos_per_plane=4)
+    spec.halos.append(synth.NFWHalo(3e13, 0.4, 0.7, 6.0))
+    return plain, glb.lens_from_spec(spec)
+
+
+@pytest.mark.parametrize("block", [64, 128, 256])
+@pytest.mark.parametrize("graph", [False, True])
+def test_batched_lenses_do_not_depend_on_each_other(block, graph):
+    """FP64 batches: lenses with and without NFW haloes in one batch have the bits
+    that they have in batches of their own; those without, the lens path's terms."""
+    plain, nfw = _mixed_lenses()
+    order = [plain[0], nfw, plain[1], nfw]
+    sides, rng = [33, 20, 64, 7], 40 * synth.ARCSEC
+    b = glb.GridBatch(order, sides, [(0.0, 0.0)] * 4, [rng] * 4, glb.PREC_FP64)
+    b.set_block(block)
+    b.run(graph)
+    for i, (lens, side) in enumerate(zip(order, sides)):
+        one = glb.GridBatch([lens], [side], [(0.0, 0.0)], [rng], glb.PREC_FP64)
+        one.run(False)
+        (y, A), (y1, A1) = b.result(i), one.result(0)
+        assert np.array_equal(y, y1) and np.array_equal(A, A1)
+        g = glb.GridMap(lens, side, (0.0, 0.0), rng, glb.PREC_FP64)
+        assert np.abs(y - g.y).max() <= 1e-11 * np.abs(g.y).max()
+        if lens is not nfw:
+            assert np.abs(A - g.A).max() <= 1e-8 * np.abs(g.A).max()
+
+
+def test_served_models_do_not_depend_on_each_other():
+    plain, nfw = _mixed_lenses()
+    x = np.random.default_rng(32).normal(0, 10 * synth.ARCSEC, (500, 2))
+    both = glb.Server([plain[0], nfw, plain[1]], precision=glb.PREC_FP64)
+    tickets = [both.submit(k, x[: 500 - 7 * k], 2.0) for k in (2, 1, 0, 1, 2)]
+    got = [both.wait(t)[:2] for t in tickets]
+    both.close()
+    for k, (y, A) in zip((2, 1, 0, 1, 2), got):
+        own = glb.Server([[plain[0], nfw, plain[1]][k]], precision=glb.PREC_FP64)
+        y1, A1 = own.wait(own.submit(0, x[: 500 - 7 * k], 2.0))[:2]
+        own.close()
+        assert np.array_equal(y, y1) and np.array_equal(A, A1)
