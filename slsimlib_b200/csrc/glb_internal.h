@@ -10,6 +10,9 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <cmath>
+#include <cstring>
+
 #include "cosmology.h"
 
 namespace glb {
@@ -87,11 +90,24 @@ struct __align__(16) FNodeS {
 // Shared walks (several warps per 32 rays) start at multiples of kCutStep nodes.
 constexpr int kCutStep = 16;
 
-// Tables of the strip walk's exponential: exp(-j/1024) and exp(-m).
-constexpr int kExpHi = 704;
-struct ExpTab {
-  double lo[1024], hi[kExpHi];
+// Table of the strip walk's exponential: 2^(-j/512) rounded to double, 2048 j added
+// to its high word, and the rounding's error over it.
+struct __align__(16) ExpTab {
+  double2 t[512];
 };
+inline ExpTab make_exp_table() {
+  ExpTab E;
+  for (int j = 0; j < 512; ++j) {
+    const long double v = exp2l(-(long double)j / 512);
+    const double h = (double)v;
+    unsigned long long b;
+    memcpy(&b, &h, 8);
+    b += (unsigned long long)(2048 * j) << 32;
+    memcpy(&E.t[j].x, &b, 8);
+    E.t[j].y = (double)((v - (long double)h) / v);
+  }
+  return E;
+}
 
 struct TreeDev {
   const TNode *tnodes;

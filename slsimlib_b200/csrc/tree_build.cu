@@ -468,12 +468,9 @@ __global__ void k_emit_nodes(const Slot *s, int nslots, double theta, GNode *nod
   cnodes[b.pre] = c;
 }
 
-// The ancestors of every kCutStep-th node, outermost first, and the tables of
-// the strip walk's exponential.
-__global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc, ExpTab *E) {
+// The ancestors of every kCutStep-th node, outermost first.
+__global__ void k_cut_ancestors(const TNode *t, int ncut, int *anc) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < 1024) E->lo[g] = exp(-(double)g / 1024.0);
-  if (g < kExpHi) E->hi[g] = exp(-(double)g);
   if (g >= ncut) return;
   const int s = g * kCutStep;
   int *a = anc + (size_t)kMaxDepth * g, k = 0, node = 0;
@@ -781,7 +778,9 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   ExpTab *exptab = (ExpTab *)(nm + o_e);
   k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes,
                                                   cnodes, fsnodes);
-  k_cut_ancestors<<<nblk(std::max(ncut, 1024), 128), 128, 0, st>>>(tnodes, ncut, cutanc, exptab);
+  if (ncut > 0) k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(tnodes, ncut, cutanc);
+  static const ExpTab exp_table = make_exp_table();
+  CK(cudaMemcpyAsync(exptab, &exp_table, sizeof(ExpTab), cudaMemcpyHostToDevice, st));
   ABuf<int> dbad(st, &arena);
   CK(dbad.alloc(1));
   CK(cudaMemsetAsync(dbad.p, 0, sizeof(int), st));
