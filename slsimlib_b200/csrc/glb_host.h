@@ -37,11 +37,11 @@ struct Status {
 inline thread_local size_t alloc_limit = 0;
 inline bool alloc_refused(size_t bytes) { return alloc_limit && bytes > alloc_limit; }
 
-// Gives back to the device what its scratch pool holds unused.
-void trim_scratch_pool();
+// Gives back to the device what its scratch pools hold unused.
+void trim_scratch_pools();
 
 // Device memory owned by RAII.  An allocation that finds no memory is tried
-// again once the scratch pool has given back what it keeps.  After a refused allocation the buffer is empty
+// again once the scratch pools have given back what they keep.  After a refused allocation the buffer is empty
 // and the runtime's last error is cleared (the caller has the status).
 template <typename T>
 struct DBuf {
@@ -61,7 +61,7 @@ struct DBuf {
     if (count == 0) return cudaSuccess;
     cudaError_t e = try_alloc(count);
     if (e == cudaErrorMemoryAllocation) {
-      trim_scratch_pool();
+      trim_scratch_pools();
       e = try_alloc(count);
     }
     if (e == cudaSuccess) n = count;
@@ -80,13 +80,16 @@ struct DBuf {
   }
 };
 
-// The pool of this device's scratch memory (tree builds, shared walks).  It
-// keeps up to 256 MB between uses, so that building many trees does not map
-// memory for each (a build takes some twenty buffers); what it holds beyond that
-// goes back to the device at the next synchronisation.
-cudaError_t scratch_pool(cudaMemPool_t *pool);
+// The pools of this device's scratch memory.  Each keeps up to 256 MB between
+// uses, so that building many trees does not map memory for each (a build takes
+// some twenty buffers); what it holds beyond that goes back to the device at the
+// next synchronisation.  Shared walks have a pool of their own: among the blocks
+// that builds leave behind, their 12 to 113 MB in one piece were mapped again by
+// every call (81 rays 1.28 ms for 1.25).
+enum ScratchKind { kBuildScratch, kWalkScratch, kScratchKinds };
+cudaError_t scratch_pool(cudaMemPool_t *pool, ScratchKind kind);
 
-// Scratch memory from the pool, taken and given back in the order of a stream.
+// Scratch memory from a pool, taken and given back in the order of a stream.
 // An arena is one such allocation that later ones carve their buffers from while
 // it has room (a small tree's twenty buffers take longer to allocate than to
 // fill).
@@ -96,8 +99,10 @@ struct ABuf {
   size_t n = 0;
   cudaStream_t s;
   struct Arena *arena;
+  ScratchKind kind = kBuildScratch;
   bool carved = false;
   explicit ABuf(cudaStream_t st, Arena *a = nullptr) : s(st), arena(a) {}
+  ABuf(cudaStream_t st, ScratchKind k) : s(st), arena(nullptr), kind(k) {}
   ABuf(const ABuf &) = delete;
   ABuf &operator=(const ABuf &) = delete;
   ~ABuf() { release(); }
@@ -132,7 +137,7 @@ cudaError_t ABuf<T>::alloc(size_t count) {
       return cudaSuccess;
     }
   cudaMemPool_t pool;
-  cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation : scratch_pool(&pool);
+  cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation : scratch_pool(&pool, kind);
   if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);
   if (e == cudaSuccess) {
     n = count;

@@ -1560,7 +1560,7 @@ const glb_halo *single_tree(const glb_lens *l, int j) {
 }
 
 // The scratch of shared walks: [sums of the parts][counters][used flags], from
-// the device's scratch pool in the order of the call's stream, so that calls on
+// the device's pool for it in the order of the call's stream, so that calls on
 // several streams neither wait for one another nor stall the device.
 constexpr int kPartCounters = 256;  // launches between two clearings of the counters
 size_t parts_bytes(size_t n, int parts, int comps) {
@@ -1712,7 +1712,7 @@ int rayshoot_device(glb_lens *l, LensWS *w, size_t n, const double *x, const dou
   // shared walks (plane_parts_max: calls of one slab);
   // without memory for their scratch the walks are not shared
   size_t psums = d_counts ? 0 : parts_sums(l, n, precision);
-  ABuf<char> parts(s);
+  ABuf<char> parts(s, kWalkScratch);
   if (psums) {
     const size_t pb = psums + parts_bytes(n, 0, 0) + psums / (5 * sizeof(double)) + 256;  // sums, counters, flags
     if (parts.alloc(pb) != cudaSuccess) psums = 0;
@@ -1886,7 +1886,7 @@ static int force_particles(const TreeDev &T, double theta, cudaStream_t s, size_
   const size_t o_perm = o_k + al(8 * n), o_bb = o_perm + al(8 * n), o_tmp = o_bb + 256, o_part = o_tmp + al(tb);
   const size_t sums = (size_t)p.nparts * 6 * n * sizeof(double);
   const size_t need = o_part + (p.nparts > 1 ? parts_bytes(n, p.nparts, 6) : 0);
-  ABuf<char> ws(s);
+  ABuf<char> ws(s, kWalkScratch);
   if (ws.alloc(need) != cudaSuccess) {
     p.nparts = 1;  // no memory for shared walks
     CKR(ws.alloc(o_part));
@@ -2023,7 +2023,7 @@ int glb_tree_force_device(glb_tree *t, size_t n, const double *rays_dev, double 
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (p.nparts > 1) CKR(cudaStreamIsCapturing(s, &cap));
     // without memory for the scratch the walks are not shared
-    ABuf<char> ws(s);
+    ABuf<char> ws(s, kWalkScratch);
     if (p.nparts > 1 && cap == cudaStreamCaptureStatusNone && ws.alloc(parts_bytes(n, p.nparts, 5)) == cudaSuccess) {
       p.px = rays_dev;
       p.py = rays_dev + 1;

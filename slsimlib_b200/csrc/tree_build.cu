@@ -554,33 +554,36 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
-void trim_scratch_pool() {
-  cudaMemPool_t pool;
-  if (scratch_pool(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+void trim_scratch_pools() {
+  for (int k = 0; k < kScratchKinds; ++k) {
+    cudaMemPool_t pool;
+    if (scratch_pool(&pool, (ScratchKind)k) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  }
   (void)cudaGetLastError();
 }
 
-cudaError_t scratch_pool(cudaMemPool_t *pool) {
+cudaError_t scratch_pool(cudaMemPool_t *pool, ScratchKind kind) {
   static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
+  static cudaMemPool_t pools[kScratchKinds][64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(mu);
-  if (!pools[dev]) {
+  cudaMemPool_t &p = pools[kind][dev];
+  if (!p) {
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    e = cudaMemPoolCreate(&pools[dev], &props);
+    e = cudaMemPoolCreate(&p, &props);
     if (e != cudaSuccess) return e;
     unsigned long long keep = 256ull << 20;
-    e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) return e;
   }
-  *pool = pools[dev];
+  *pool = p;
   return cudaSuccess;
 }
 

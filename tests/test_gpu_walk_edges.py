@@ -441,3 +441,19 @@ def test_served_models_do_not_depend_on_each_other():
         y1, A1 = own.wait(own.submit(0, x[: 500 - 7 * k], 2.0))[:2]
         own.close()
         assert np.array_equal(y, y1) and np.array_equal(A, A1)
+
+
+def test_small_calls_after_builds_map_no_memory():
+    """Trees built and freed leave their pool in pieces; the scratch of a small
+    call is not mapped and given back by each call for that."""
+    import torch
+    lens = _lens(400000)
+    x = np.random.default_rng(33).normal(0, 10 * synth.ARCSEC, (4097, 2))
+    for n in (50000, 300000, 150000):
+        glb.TreeQuadParticles(_cluster(n, n), bucket=5, theta_force=0.1)
+    want = lens.rayshooterInternal(x)
+    free = torch.cuda.mem_get_info()[0]
+    for again in range(3):
+        got = lens.rayshooterInternal(x)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        assert torch.cuda.mem_get_info()[0] == free
