@@ -113,6 +113,9 @@ struct ABuf {
     carved = false;
   }
   cudaError_t alloc(size_t count);
+
+ private:
+  cudaError_t try_alloc(size_t count);
 };
 struct Arena {
   ABuf<char> mem;
@@ -136,6 +139,13 @@ cudaError_t ABuf<T>::alloc(size_t count) {
       carved = true;
       return cudaSuccess;
     }
+  const cudaError_t e0 = try_alloc(count);
+  if (e0 != cudaErrorMemoryAllocation) return e0;
+  trim_scratch_pools();
+  return try_alloc(count);
+}
+template <typename T>
+cudaError_t ABuf<T>::try_alloc(size_t count) {
   cudaMemPool_t pool;
   cudaError_t e = alloc_refused(count * sizeof(T)) ? cudaErrorMemoryAllocation : scratch_pool(&pool, kind);
   if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), pool, s);

@@ -457,3 +457,15 @@ def test_small_calls_after_builds_map_no_memory():
         got = lens.rayshooterInternal(x)
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
         assert torch.cuda.mem_get_info()[0] == free
+
+
+@pytest.mark.parametrize("bucket", [5, 20])
+def test_builds_without_their_scratch_in_one_piece(bucket):
+    """Where the one piece (over 240 bytes a particle) cannot be had, a build goes on
+    with the buffers' own allocations."""
+    p = _cluster(34, 100000)
+    x = np.random.default_rng(35).normal(0, 0.3, (500, 2))
+    want = _recur(glb.TreeQuadParticles(p, bucket=bucket, theta_force=0.1), x)
+    with alloc_limit((1 << 20) + 240 * len(p)):
+        t = glb.TreeQuadParticles(p, bucket=bucket, theta_force=0.1)
+    assert np.array_equal(_recur(t, x), want)
