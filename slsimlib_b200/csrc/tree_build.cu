@@ -703,8 +703,10 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   const int nslots = off[nlev];
 
   // ---- moments, bottom-up
-  CK(T->particles.alloc(2 * n));
-  float4 *parts = T->particles.p, *prel = parts + n;
+  const bool pieces = in_pieces(n * sizeof(float4), n * sizeof(float4));
+  CK(T->particles.alloc(pieces ? n : 2 * n));
+  if (pieces) CK(T->particles_more.alloc(n));
+  float4 *parts = T->particles.p, *prel = pieces ? T->particles_more.p : parts + n;
   for (int L = nlev - 1; L >= 0; --L) {
     int lo = off[L], hi = off[L + 1];
     k_leaf_moments<<<nblk((long long)(hi - lo) * 32, 256), 256, 0, st>>>(slots.p, lo, hi, dp.p, sidx.p, multimass,
@@ -767,20 +769,23 @@ Status build_tree(const glb_particle_rec *hp, size_t n, const TreeParams &prm, b
   // ---- node array
   const int ncut = (nnodes + kCutStep - 1) / kCutStep;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t nn = (size_t)nnodes, o_g = 0, o_s = o_g + al(nn * sizeof(GNode)), o_t = o_s + al(nn * sizeof(GNodeS));
-  const size_t o_f = o_t + al(nn * sizeof(TNode)), o_n = o_f + al(nn * sizeof(FNode));
+  const size_t nn = (size_t)nnodes, o_g = 0, o_s = o_g + al(nn * sizeof(GNode)), half = o_s + al(nn * sizeof(GNodeS));
+  const size_t o_t = 0, o_f = o_t + al(nn * sizeof(TNode)), o_n = o_f + al(nn * sizeof(FNode));
   const size_t o_r = o_n + al(nn * sizeof(CNode)), o_c = o_r + al(nn * sizeof(FNodeS));
   const size_t o_e = o_c + al((size_t)ncut * kMaxDepth * sizeof(int));
-  CK(T->node_mem.alloc(o_e + sizeof(ExpTab)));
-  char *nm = T->node_mem.p;
+  const size_t rest = o_e + sizeof(ExpTab);
+  const bool two = in_pieces(half, rest);
+  CK(T->node_mem.alloc(two ? half : half + rest));
+  if (two) CK(T->node_more.alloc(rest));
+  char *nm = T->node_mem.p, *nm2 = two ? T->node_more.p : nm + half;
   GNode *gnodes = (GNode *)(nm + o_g);
   GNodeS *snodes = (GNodeS *)(nm + o_s);
-  TNode *tnodes = (TNode *)(nm + o_t);
-  FNode *fnodes = (FNode *)(nm + o_f);
-  CNode *cnodes = (CNode *)(nm + o_n);
-  FNodeS *fsnodes = (FNodeS *)(nm + o_r);
-  int *cutanc = (int *)(nm + o_c);
-  ExpTab *exptab = (ExpTab *)(nm + o_e);
+  TNode *tnodes = (TNode *)(nm2 + o_t);
+  FNode *fnodes = (FNode *)(nm2 + o_f);
+  CNode *cnodes = (CNode *)(nm2 + o_n);
+  FNodeS *fsnodes = (FNodeS *)(nm2 + o_r);
+  int *cutanc = (int *)(nm2 + o_c);
+  ExpTab *exptab = (ExpTab *)(nm2 + o_e);
   k_emit_nodes<<<nblk(nslots, 256), 256, 0, st>>>(slots.p, nslots, prm.theta, gnodes, snodes, tnodes, fnodes,
                                                   cnodes, fsnodes);
   if (ncut > 0) k_cut_ancestors<<<nblk(ncut, 128), 128, 0, st>>>(tnodes, ncut, cutanc);

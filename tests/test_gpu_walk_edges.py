@@ -469,3 +469,18 @@ def test_builds_without_their_scratch_in_one_piece(bucket):
     with alloc_limit((1 << 20) + 240 * len(p)):
         t = glb.TreeQuadParticles(p, bucket=bucket, theta_force=0.1)
     assert np.array_equal(_recur(t, x), want)
+
+
+@pytest.mark.parametrize("n", [16384, 32768, 32769, 36000, 65536, 65537])
+def test_trees_at_the_edges_of_their_allocations(n):
+    """Particles and nodes lie in one allocation or two (1 MB): forces of every form
+    against the oracle (the split form's within its 1e-5 at the 99.9th percentile)."""
+    from tests import harness as H
+    from tests.test_gpu_parity import force_err, pack, vec_err
+    p = _cluster(n, n, 0.002)
+    x = np.random.default_rng(36).normal(0, 0.3, (1000, 2))
+    t = glb.TreeQuadParticles(p, bucket=20, theta_force=0.1, inv_screening_scale=1.0)
+    want = H.OracleTree(p, bucket=20, theta=0.1, inv_area=0.0, inv_screening=1.0, periodic=0).force(x[:100])
+    assert force_err(pack(*t.force2D_recur(x[:100])), want)[0] < 1e-9
+    fp64, split = _device_force(t, x), _device_force(t, x, glb.PREC_SPLIT)
+    assert np.quantile(vec_err(split[:, :2], fp64[:, :2]), 0.999) < 1e-5
