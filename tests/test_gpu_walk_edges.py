@@ -484,3 +484,41 @@ def test_trees_at_the_edges_of_their_allocations(n):
     assert force_err(pack(*t.force2D_recur(x[:100])), want)[0] < 1e-9
     fp64, split = _device_force(t, x), _device_force(t, x, glb.PREC_SPLIT)
     assert np.quantile(vec_err(split[:, :2], fp64[:, :2]), 0.999) < 1e-5
+
+
+def _signed(seed, n, size):
+    p = _cluster(seed, n, size)
+    p["Mass"] *= np.where(np.random.default_rng(seed + 100).random(n) < 0.3, -1e9, 1e9).astype(np.float32)
+    return p
+
+
+@pytest.mark.parametrize("n", [200, 70000, 131072])
+def test_two_particle_haloes_on_one_plane(n):
+    """FP64 planes with two particle haloes (the kernel without a tree in its
+    parameters) against the oracle."""
+    from tests import harness as H
+    spec = synth.LensSpec(zsource=2.0, halos=[
+        synth.ParticlePlane(_signed(40, 3000, 0.02), 0.3, inv_area=0.0), synth.ParticlePlane(_cluster(41, 500, 0.05), 0.3),
+        synth.ParticlePlane(_signed(42, 2000, 0.01), 0.7)])
+    lens = glb.lens_from_spec(spec)
+    assert lens.getNplanes() == 2
+    x = np.random.default_rng(43).normal(0, 30 * synth.ARCSEC, (n, 2))
+    y, A = lens.rayshooterInternal(x)
+    yo, Ao = H.OracleLens(spec).rayshoot(x[:200])
+    assert np.abs(y[:200] - yo).max() < 1e-9 * np.abs(yo).max()
+    assert np.abs(A[:200] - Ao).max() < 1e-8 * np.abs(Ao).max()
+
+
+@pytest.mark.parametrize("inv_area", [0.0, 0.3])
+@pytest.mark.parametrize("size", [0.001, 0.3])  # 0.3: most particles are softened at internal nodes
+def test_two_rays_per_lane_with_sheets_signs_and_softening(inv_area, size):
+    lens = glb.Lens(2.0)
+    for z, s in ((0.3, 50), (0.8, 51)):
+        lens.insertMainHalo(glb.LensHaloParticles(_signed(s, 8000, size), z, inv_area=inv_area), True)
+    x = np.random.default_rng(52).normal(0, 40 * synth.ARCSEC, (131072, 2))
+    zs = np.random.default_rng(53).uniform(0.05, 3.0, len(x))
+    for z in (None, zs):
+        y, A = lens.rayshooterInternal(x, z)  # two rays per lane
+        assert np.all(np.isfinite(A))
+        ys, As = lens.rayshooterInternal(x[:66049], None if z is None else z[:66049])  # one
+        assert np.array_equal(y[:66049], ys) and np.array_equal(A[:66049], As)
