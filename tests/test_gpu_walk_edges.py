@@ -522,3 +522,24 @@ def test_two_rays_per_lane_with_sheets_signs_and_softening(inv_area, size):
         assert np.all(np.isfinite(A))
         ys, As = lens.rayshooterInternal(x[:66049], None if z is None else z[:66049])  # one
         assert np.array_equal(y[:66049], ys) and np.array_equal(A[:66049], As)
+
+
+@pytest.mark.parametrize("n", [100, 70001])
+def test_two_large_particle_haloes_on_one_plane(n):
+    """A tree of more than 2^18 nodes beside another on a plane: node by node, the
+    terms of the two haloes on planes (nearly) of their own."""
+    p, q = _cluster(60, 2000000, 0.0005), _cluster(61, 3000, 0.01)
+    for c in (p, q):
+        c["Mass"] *= 1e9
+    x = np.random.default_rng(62).normal(0, 60 * synth.ARCSEC, (n, 2))
+    both, one, two = glb.Lens(2.0), glb.Lens(2.0), glb.Lens(2.0)
+    both.insertMainHalo(glb.LensHaloParticles(p, 0.3), True)
+    both.insertMainHalo(glb.LensHaloParticles(q, 0.3), True)
+    one.insertMainHalo(glb.LensHaloParticles(p, 0.3), True)
+    two.insertMainHalo(glb.LensHaloParticles(q, 0.3), True)
+    assert both.getNplanes() == 1
+    (y, A), (y1, A1), (y2, A2) = (lens.rayshooterInternal(x) for lens in (both, one, two))
+    # one plane: deflections and the Jacobian's deviations from unity add up
+    assert np.abs(y - (y1 + y2 - x)).max() <= 1e-11 * np.abs(y).max()
+    unit = np.array([1.0, 0.0, 0.0, 1.0])
+    assert np.abs(A - (A1 + A2 - unit)).max() <= 1e-10 * np.abs(A).max()
