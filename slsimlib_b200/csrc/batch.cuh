@@ -143,7 +143,7 @@ __device__ __forceinline__ void plane_force(const PlaneDev &P, const HaloDev *ha
 }
 template <int PREC>
 // The list and strip forms take 128 registers (2 blocks of 256 per SM): 48 uneven
-// lenses, list form, 70.3 ms; with 80 registers 90.  The node-at-a-time forms take
+// lenses, list form, 70 ms; with 80 registers 90.  The node-at-a-time forms take
 // 80, for occupancy (64 registers measured slower there).
 // dynamic shared memory: batch_smem_bytes(blockDim.x)
 __global__ void __launch_bounds__(256, PREC == kListForm || PREC == kStripForm ? 2 : 3) k_batch(const Chunk *chunks, int nchunks, const LensDev *lenses,

@@ -1566,8 +1566,8 @@ constexpr int kPartCounters = 256;  // launches between two clearings of the cou
 size_t parts_bytes(size_t n, int parts, int comps) {
   return (size_t)parts * comps * n * sizeof(double) + kPartCounters * sizeof(int) + (size_t)parts * ((n + 31) / 32);
 }
-// Points p at scratch for launch number i of a pass (its counter cleared by
-// clear_part_counters).
+// Points p at scratch for launch number i of a pass (its counter was cleared at the
+// last multiple of kPartCounters).
 void set_part_scratch(PartArgs &p, char *scratch, size_t sums, int i) {
   p.out = (double *)scratch;
   p.counter = (int *)(scratch + sums) + i % kPartCounters;
@@ -1597,6 +1597,13 @@ size_t parts_sums(const glb_lens *l, size_t n, int precision) {
   return m;
 }
 
+// Planes with several particle haloes, whose walks are not shared, take strips up
+// to this many nodes: two haloes of 72,000 nodes each, 102,400 rays over 10 and 90
+// arcsec, node by node / strips 17.0 / 14.4, 21.7 / 18.7 ms; of 289,000 nodes 22.3 /
+// 26.3, 38.1 / 40.0.
+constexpr int kStripPlaneMax = 1 << 18;
+constexpr size_t kTwoRayMin = (size_t)1 << 20;  // two-ray tree-force kernel from this many rays on
+
 // One launch per plane, in order.  Split-form planes that hold exactly one
 // particle halo and no field plane run the group walk (k_plane_step_split_g,
 // the tree in the kernel parameters); planes with a field plane use the FIELD
@@ -1605,14 +1612,8 @@ size_t parts_sums(const glb_lens *l, size_t n, int precision) {
 // bin cancel up to 1e9-fold (nfw_g, nfw_g2), so a ray that meets a halo's
 // centre carries the last bit of its position into the ninth digit of A, and
 // those lenses keep the walk whose last bits are the reference's operations.
-// Small FP64 calls share their walks (strip_parts) where the caller has scratch
-// for them (parts_sums).
-// Planes with several particle haloes, whose walks are not shared, take strips up
-// to this many nodes: two haloes of 72,000 nodes each, 102,400 rays over 10 and 90
-// arcsec, node by node / strips 17.0 / 14.4, 21.7 / 18.7 ms; of 289,000 nodes 22.3 /
-// 26.3, 38.1 / 40.0.
-constexpr int kStripPlaneMax = 1 << 18;
-constexpr size_t kTwoRayMin = (size_t)1 << 20;  // two-ray tree-force kernel from this many rays on
+// FP64 calls of few rays (plane_parts_max) share their walks (strip_parts) where the
+// caller has scratch for them (parts_sums).
 int launch_plane_steps(const glb_lens *l, StepArgs &a, int jmax_launch, int precision, cudaStream_t s,
                        const unsigned long long *d_counts, char *scratch = nullptr, size_t sums = 0) {
   const size_t n = a.n;

@@ -12,7 +12,7 @@
 // walked per ray.  A node-at-a-time walk tests about 5,200 cells per ray here;
 // this one about 4,300 cells in rounds of 32, and per ray only the nodes of
 // mixed subtrees.  48 uneven lenses in one launch (2.8M rays): 89 ms with the
-// node-at-a-time walk, 72.9 with this one; 16 served requests 57 and 39 ms.
+// node-at-a-time walk, 70 with this one; 16 served requests 57 and 41 ms.
 #pragma once
 #include "walk_group.cuh"
 #include "walk_strip.cuh"
@@ -140,7 +140,7 @@ __device__ __forceinline__ void walk_list(const TreeDev &T, double rx, double ry
     list_classify(T, w, L, nwait, w0, w1);
 #pragma unroll 1
     for (int h = 0; h < kLW / 1024; ++h) {
-      // the half window's cells in order: offset | category << kLBits
+      // a quarter window's cells in order: offset | category << kLBits
       const unsigned f = L.far[32 * h + w.lane], e = L.open[32 * h + w.lane], m = L.mixed[32 * h + w.lane];
       unsigned all = f | e;
       if (!__any_sync(kFull, all != 0u)) continue;

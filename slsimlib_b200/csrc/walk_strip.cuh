@@ -29,12 +29,14 @@
 // node-at-a-time walk (walk_f64) adds them, so its sums do not depend on the
 // other rays and stay within a few roundings of that walk's.
 //
-// Bound by FP64 latency and issue: 512^2 rays on 2^18 particles take 7.9 ms
-// (12.9 with walk_f64), 2.6 of them in far-field terms (76 % of the FP64 pipe's
-// rate), 2.4 in particles, 1.8 in the exponentials of both, 2.1 in strips and
-// staging; FP64 pipe 48 %, issue 61 % at 18 warps per SM (96 registers; 80 or
-// 128 registers and loops unrolled by 2 within 3 % of it, unrolled by 4 13.3
-// ms: the instruction cache).
+// Bound by FP64 latency and issue: 512^2 rays on 2^18 particles take 12.9 ms with
+// walk_f64, 7.9 with one ray per lane (96 registers, 18 warps per SM), 7.0 with two
+// (128 registers, 14 warps; FP64 pipe and issue 57 %).  Of the 7.9, 2.6 are far-field
+// terms (76 % of the FP64 pipe's rate), 2.4 particles, 1.8 the exponentials of both,
+// 2.1 strips and staging; 80 or 128 registers and loops unrolled by 2 are within 3 %
+// of it, unrolled by 4 13.3 ms (the instruction cache).  Where most nodes of a strip
+// are mixed (few rays in a large tree, small leaves, wide opening angles) walk_f64
+// is the faster one: force_rule, host_force_rule and plane_parts_max draw the line.
 #pragma once
 #include "walk.cuh"
 
