@@ -80,13 +80,16 @@ struct DBuf {
   }
 };
 
-// The pools of this device's scratch memory.  Each keeps up to 256 MB between
-// uses, so that building many trees does not map memory for each (a build takes
-// some twenty buffers); what it holds beyond that goes back to the device at the
-// next synchronisation.  Shared walks have a pool of their own: among the blocks
-// that builds leave behind, their 12 to 113 MB in one piece were mapped again by
-// every call (81 rays 1.28 ms for 1.25).
+// The pools of this device's scratch memory.  Each keeps what it was at most asked
+// for at once, up to kScratchKept, between uses, so that building many trees does
+// not map memory for each (a build takes some twenty buffers); what it holds beyond
+// that goes back to the device at the next synchronisation.  Shared walks have a
+// pool of their own: among the blocks that builds leave behind, their 12 to 113 MB
+// in one piece were mapped again by every call (81 rays 1.28 ms for 1.25); and its
+// limit holds a dozen calls at once (eight threads, 4,097 rays each: 0.8 ms a call,
+// 0.8 to 1.5 with 256 MB).
 enum ScratchKind { kBuildScratch, kWalkScratch, kScratchKinds };
+constexpr unsigned long long kScratchKept[kScratchKinds] = {256ull << 20, 1024ull << 20};
 cudaError_t scratch_pool(cudaMemPool_t *pool, ScratchKind kind);
 
 // Scratch memory from a pool, taken and given back in the order of a stream.

@@ -579,7 +579,7 @@ cudaError_t scratch_pool(cudaMemPool_t *pool, ScratchKind kind) {
     props.location.id = dev;
     e = cudaMemPoolCreate(&p, &props);
     if (e != cudaSuccess) return e;
-    unsigned long long keep = 256ull << 20;
+    unsigned long long keep = kScratchKept[kind];
     e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) return e;
   }

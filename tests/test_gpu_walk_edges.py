@@ -543,3 +543,25 @@ def test_two_large_particle_haloes_on_one_plane(n):
     assert np.abs(y - (y1 + y2 - x)).max() <= 1e-11 * np.abs(y).max()
     unit = np.array([1.0, 0.0, 0.0, 1.0])
     assert np.abs(A - (A1 + A2 - unit)).max() <= 1e-10 * np.abs(A).max()
+
+
+def test_the_scratch_of_calls_at_once_is_kept():
+    """Eight calls in flight on eight streams hold 80 MB each; the pool keeps them for
+    the next eight instead of mapping memory for each call."""
+    import torch
+    t = glb.TreeQuadParticles(_cluster(63, 200000), bucket=5, theta_force=0.05)
+    x = np.random.default_rng(64).normal(0, 0.3, (5000, 2))
+    want = _device_force(t, x)
+    lens = _lens()
+    with alloc_limit(1 << 20):
+        _refused(lambda: lens.rayshooterInternal(np.zeros((60000, 2))))  # gives back what the pools hold
+    d = torch.from_numpy(x).cuda()
+    out = torch.zeros((8, len(x), 5), dtype=torch.float64, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(8)]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for o, s in zip(out, streams):
+        t.force_device(len(x), d.data_ptr(), o.data_ptr(), glb.PREC_FP64, s.cuda_stream)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] > 500 << 20
+    assert all(np.array_equal(o, want) for o in out.cpu().numpy())
